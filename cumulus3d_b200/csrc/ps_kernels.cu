@@ -12,9 +12,8 @@
 //
 // The rules are those of the reference kernel crates/cuda/src/kernels/patchmatch.cu (cited per function) and of
 // crates/dense/src/kernel.rs:36-74.  The B200 layout differs from the reference:
-//   * every image level is a normalised f32 plane with a PS_BORDER-pixel zero border, so a bilinear source tap is
-//     four unconditional loads after a clamp (no per-texel bounds tests); optionally (PS_TUNE_TEX_GATHER) a gather
-//     through a border-addressed texture fetches the same four texels with one instruction;
+//   * every image level is a normalised f32 plane with a PS_BORDER-pixel zero border (reference tiles, TMA boxes) and a
+//     border-addressed texture of the same values: one gather fetches the four texels of a bilinear source tap;
 //   * a half-step CTA is 128 threads covering a 32 × 8 pixel tile; each warp takes 16 active columns of two
 //     adjacent rows, so reference-tile reads of the two colour phases fall into disjoint shared-memory banks;
 //   * the bilateral window weights of a pixel are computed once per half step and cached in shared memory (one
@@ -140,37 +139,10 @@ __device__ __forceinline__ float3 pixel_ray(const PsLevel& R, int x, int y) {
 }
 
 // ------------------------------------------------------------------------------------------- source sample (patchmatch.cu:169-192)
-// Bilinear value at (u, v), integer-centre convention, 0 outside the image.  The clamp to [-2, w] × [-2, h] keeps
-// both taps of an out-of-image footprint inside the zero border, which reproduces the reference's "0 outside"
-// without per-texel tests.
-__device__ __forceinline__ int f2i_exact(float v) {
-  // v is an integer in [-2^22, 2^22]: adding 1.5·2^23 puts it in the low mantissa bits (one FADD instead of the
-  // quarter-rate F2I conversion).
-  return __float_as_int(v + 12582912.0f) - 0x4B400000;
-}
-__device__ __forceinline__ float src_sample(const float* __restrict__ img, int pitch, float wf, float hf, float u,
-                                            float v, unsigned long long* fault = nullptr) {
-  float xf = floorf(u), yf = floorf(v);
-  float ax = u - xf, ay = v - yf;
-  float xc = fminf(fmaxf(xf, -2.0f), wf);
-  float yc = fminf(fmaxf(yf, -2.0f), hf);
-#if PS_CHECKED
-  // the 2 × 2 footprint inside the bordered plane: columns [-PS_BORDER, pitch - PS_BORDER), rows [-PS_BORDER,
-  // h + PS_BORDER)
-  if (!PS_IN(fault, PS_SITE_PLANE, f2i_exact(xc), -PS_BORDER, pitch - PS_BORDER - 1) ||
-      !PS_IN(fault, PS_SITE_PLANE, f2i_exact(yc), -PS_BORDER, (int)hf + PS_BORDER - 1))
-    return 0.f;
-#endif
-  const float* p = img + f2i_exact(yc) * pitch + f2i_exact(xc);
-  float p00 = __ldg(p), p10 = __ldg(p + 1), p01 = __ldg(p + pitch), p11 = __ldg(p + pitch + 1);
-  float top = fmaf(ax, p10 - p00, p00);
-  float bot = fmaf(ax, p11 - p01, p01);
-  return fmaf(ay, bot - top, top);
-}
-// Same sample through the texture unit: a gather at the exact integer coordinate (x0, y0) selects the footprint
-// (x0-1 .. x0, y0-1 .. y0), and the texel offset (+1, +1) of the tld4 instruction moves it onto (x0 .. x0+1,
-// y0 .. y0+1), so the four texels come back without two coordinate additions per tap (border addressing gives 0
-// outside the image).  The bilinear arithmetic is unchanged, so the result has the same bits as src_sample.
+// Bilinear value at (u, v), integer-centre convention, 0 outside the image.  A gather at the exact integer coordinate
+// (x0, y0) selects the footprint (x0-1 .. x0, y0-1 .. y0), and the texel offset (+1, +1) of the tld4 instruction moves
+// it onto (x0 .. x0+1, y0 .. y0+1), so the four texels come back without two coordinate additions per tap (border
+// addressing gives 0 outside the image); the bilinear arithmetic is in binary32 registers.
 // Gather order: (T[x0,y1], T[x1,y1], T[x1,y0], T[x0,y0]).
 __device__ __forceinline__ float4 gather_red_offset11(unsigned long long tex, float x, float y) {
   float4 q;
@@ -179,7 +151,7 @@ __device__ __forceinline__ float4 gather_red_offset11(unsigned long long tex, fl
       : "l"(tex), "f"(x), "f"(y), "r"(1), "r"(1));
   return q;
 }
-__device__ __forceinline__ float src_sample_tex(unsigned long long tex, float u, float v) {
+__device__ __forceinline__ float src_sample(unsigned long long tex, float u, float v) {
   float xf = floorf(u), yf = floorf(v);
   float ax = u - xf, ay = v - yf;
   const float4 q = gather_red_offset11(tex, xf, yf);
@@ -194,22 +166,17 @@ struct RefStats {
   float ic, W, mu, var;
 };
 
-// Tile-resident reference window of one pixel: t points at the pixel inside the shared tile (row pitch tw); wc is
-// the thread's weight-cache slot (stride NT floats between taps).  Window sums are split by row parity: even rows
-// (a = 0, 2, …) and odd rows (a = 1, 3, …) accumulate separately, in ascending row order, and the NCC uses
-// even + odd.  With G = 2 lanes per pixel, lane g sums the rows of parity g and the two partial sums meet through
-// one shuffle (pmask = the pair's lanes); with G = 1 one thread keeps both partial sums.
+// Tile-resident reference window of one pixel: t points at the pixel inside the shared tile (row pitch tw).  Window sums
+// are split by row parity: even rows (a = 0, 2, …) and odd rows (a = 1, 3, …) accumulate separately, in ascending row
+// order, and the NCC uses even + odd.
 //
-// Weight-cache layouts: per tap (a, b) one float per thread, stride NT between taps.  The legacy layout keeps row a at
-// wc + a·wn·NT.  The row-pair layout (PW) used by the f32x2 tap loops puts the weights of rows 2p and 2p+1 of the
-// same column next to each other (one 8-byte load per tap pair): wc + (p·wn + b)·2·NT + (a & 1) with wc = base +
-// 2·thread, and the last row of an odd window at wl + b·NT.
+// Weight cache: one float per thread and tap, NT threads.  The weights of rows 2p and 2p+1 of the same column lie next to
+// each other (one 8-byte load per tap pair): wc + (p·wn + b)·2·NT + (a & 1) with wc = base + 2·thread, and the last row
+// of an odd window at wl + b·NT with wl = base + (wn & ~1)·wn·NT + thread.
 struct RefWin {
   const float* t;
   int tw;
   float* wc;
-  int g;
-  unsigned pmask;
   float* wl;
 #if PS_CHECKED
   const float* tbase;  // the tile and its size in floats
@@ -234,19 +201,15 @@ __device__ __forceinline__ float tile_at(const RefWin& rw, const float* p) {
   return *p;
 }
 
-// Row-parity partial sums -> total (even + odd; IEEE addition is commutative, so both lanes get the same bits).
-template <int G>
-__device__ __forceinline__ float pair_total(const RefWin& rw, const float* part) {
-  if constexpr (G == 1) {
-    return part[0] + part[1];
-  } else {
-    const float other = __shfl_xor_sync(rw.pmask, part[0], 1);
-    return part[0] + other;
-  }
+// The thread's weight-cache slots (see RefWin) in the cache at `cache`.
+template <int NT>
+__device__ __forceinline__ void refwin_cache(RefWin& rw, float* cache, int wn) {
+  rw.wc = cache + 2 * threadIdx.x;
+  rw.wl = cache + (wn & ~1) * wn * NT + threadIdx.x;
 }
 
 // ref_stats (patchmatch.cu:199-223).  Weights w_k = exp(-(dx²+dy²)/(2σs²) - (Ic-Ik)²/(2σc²)); 0 outside the image.
-template <int WR, int WS, bool CW, int NT, int G = 1, bool PW = false>
+template <int WR, int WS, bool CW, int NT>
 __device__ __forceinline__ RefStats ref_stats(const PsRun& P, const RefWin& rw) {
   const int wr = WR ? WR : P.wr, ws = WR ? WS : P.ws;
   const int wn = (2 * wr) / ws + 1;
@@ -254,22 +217,13 @@ __device__ __forceinline__ RefStats ref_stats(const PsRun& P, const RefWin& rw) 
   s.ic = tile_at(rw, rw.t);
   float W[2] = {0.f, 0.f}, S[2] = {0.f, 0.f}, SS[2] = {0.f, 0.f};
 #pragma unroll 1
-  for (int a = (G == 2 ? rw.g : 0); a < wn; a += G) {
+  for (int a = 0; a < wn; ++a) {
     const int dy = -wr + a * ws;
-    const int pa = G == 2 ? 0 : (a & 1);
+    const int pa = a & 1;
     const float* trow = rw.t + dy * rw.tw;
-    float* wrow;
-    int wst = NT;
-    if constexpr (PW) {
-      if (a < (wn & ~1)) {
-        wrow = rw.wc + (a >> 1) * wn * NT * 2 + (a & 1);
-        wst = 2 * NT;
-      } else {
-        wrow = rw.wl;
-      }
-    } else {
-      wrow = rw.wc + (G == 2 ? (a >> 1) : a) * wn * NT;
-    }
+    const bool paired = a < (wn & ~1);
+    float* wrow = paired ? rw.wc + (a >> 1) * wn * NT * 2 + (a & 1) : rw.wl;
+    const int wst = paired ? 2 * NT : NT;
     auto tap = [&](int b) {
       const int dx = -wr + b * ws;
       float ik = tile_at(rw, trow + dx);
@@ -289,8 +243,8 @@ __device__ __forceinline__ RefStats ref_stats(const PsRun& P, const RefWin& rw) 
       for (int b = 0; b < wn; ++b) tap(b);
     }
   }
-  s.W = pair_total<G>(rw, W);
-  const float St = pair_total<G>(rw, S), SSt = pair_total<G>(rw, SS);
+  s.W = W[0] + W[1];
+  const float St = S[0] + S[1], SSt = SS[0] + SS[1];
   s.mu = St / s.W;
   s.var = SSt / s.W - s.mu * s.mu;
   return s;
@@ -348,124 +302,17 @@ __device__ __forceinline__ float ncc_finish(const RefStats& rs, float Sst, float
   return fminf(fmaxf(c, 0.0f), 2.0f);
 }
 
-// Window sums over the taps (patchmatch.cu:263-279) and the cost; the prologue must have passed.
+// ================================================================================ row-pair tap loops (f32x2)
+// The window sums (patchmatch.cu:263-279) with rows 2p (even) and 2p+1 (odd) in the two halves of f32x2 pairs.  The
+// even-row and odd-row partial sums of the parity contract advance in the reference's tap order, so the pairing changes
+// no bits, and each pair operation takes one issue slot for two taps.  Sources are sampled by a texture gather, or in the
+// staged half step from the warp's source box (shared memory).
 //
 // A tap behind the source camera (zz <= 1e-8) samples 0.  The computed zz = fma(H6, sx, fma(H7, sy, H8)) is monotone
 // in sx for a fixed row and, through the correctly rounded inner fma, monotone in sy for a fixed column (each step is
 // a correctly rounded function of an affine expression, and rounding is monotone), so the smallest zz of the window
-// is at one of its four corner taps.  When all four are in front, every tap is, and the taps run without the
-// per-tap test and selects; otherwise a guarded loop handles each tap (the same bits either way).
-template <int WR, int WS, bool CW, int NT, bool TEX, int G, bool PW = false>
-__device__ __forceinline__ float ncc_window(const PsRun& P, const RefWin& rw, const RefStats& rs, const PsLevel& S,
-                                            const float* H, int x, int y) {
-  const int wr = WR ? WR : P.wr, ws = WR ? WS : P.ws;
-  const int wn = (2 * wr) / ws + 1;
-  const float fx = (float)x, fy = (float)y;
-  const float wf = (float)S.w, hf = (float)S.h;
-  const float* __restrict__ img = S.img;
-  const unsigned long long tex = S.tex;
-  const int pitch = S.pitch;
-  float Ss[2] = {0.f, 0.f}, SSs[2] = {0.f, 0.f}, IS[2] = {0.f, 0.f};
-  const float sx0 = fx + (float)(-wr), sx1 = fx + (float)wr;
-  const float rz0 = fmaf(H[7], fy + (float)(-wr), H[8]), rz1 = fmaf(H[7], fy + (float)wr, H[8]);
-  const bool all_front = fmaf(H[6], sx0, rz0) > 1e-8f && fmaf(H[6], sx1, rz0) > 1e-8f &&
-                         fmaf(H[6], sx0, rz1) > 1e-8f && fmaf(H[6], sx1, rz1) > 1e-8f;
-  auto sample = [&](float uf, float vf) {
-    if constexpr (TEX) return src_sample_tex(tex, uf, vf);
-    else return src_sample(img, pitch, wf, hf, uf, vf, P.fault);
-  };
-  auto accumulate = [&](int pa, float w, float sv, float ik) {
-    const float wsv = w * sv;
-    Ss[pa] = Ss[pa] + wsv;
-    SSs[pa] = fmaf(wsv, sv, SSs[pa]);
-    IS[pa] = fmaf(wsv, ik, IS[pa]);
-  };
-  // weights of row a start at wrow(a), stride wst(a) between taps (legacy or row-pair cache layout)
-  auto wrow_of = [&](int a) -> const float* {
-    if constexpr (PW) return a < (wn & ~1) ? rw.wc + (a >> 1) * wn * NT * 2 + (a & 1) : rw.wl;
-    else return rw.wc + (G == 2 ? (a >> 1) : a) * wn * NT;
-  };
-  auto wst_of = [&](int a) { return (PW && a < (wn & ~1)) ? 2 * NT : NT; };
-  auto weight = [&](const float* wrow, int wst, int b, int dx, int dy, float ik) {
-    if constexpr (CW) {
-      return wrow[b * wst];
-    } else {
-      const float d = rs.ic - ik;
-      return m_exp(-(float)(dx * dx + dy * dy) * P.inv2s - d * d * P.inv2c);
-    }
-  };
-  if (all_front) {
-#pragma unroll 1
-    for (int a = (G == 2 ? rw.g : 0); a < wn; a += G) {
-      const int dy = -wr + a * ws;
-      const int pa = G == 2 ? 0 : (a & 1);
-      const float sy = fy + (float)dy;
-      const float rx = fmaf(H[1], sy, H[2]);
-      const float ry = fmaf(H[4], sy, H[5]);
-      const float rz = fmaf(H[7], sy, H[8]);
-      const float* trow = rw.t + dy * rw.tw;
-      const float* wrow = wrow_of(a);
-      const int wst = wst_of(a);
-      auto tap = [&](int b) {
-        const int dx = -wr + b * ws;
-        const float sx = fx + (float)dx;
-        const float ik = tile_at(rw, trow + dx);
-        const float w = weight(wrow, wst, b, dx, dy, ik);
-        const float izz = m_rcp(fmaf(H[6], sx, rz));
-        accumulate(pa, w, sample(fmaf(H[0], sx, rx) * izz, fmaf(H[3], sx, ry) * izz), ik);
-      };
-      if constexpr (WR != 0) {
-#pragma unroll
-        for (int b = 0; b < (2 * WR) / WS + 1; ++b) tap(b);
-      } else {
-#pragma unroll 1
-        for (int b = 0; b < wn; ++b) tap(b);
-      }
-    }
-  } else {
-#pragma unroll 1
-    for (int a = (G == 2 ? rw.g : 0); a < wn; a += G) {
-      const int dy = -wr + a * ws;
-      const int pa = G == 2 ? 0 : (a & 1);
-      const float sy = fy + (float)dy;
-      const float rx = fmaf(H[1], sy, H[2]);
-      const float ry = fmaf(H[4], sy, H[5]);
-      const float rz = fmaf(H[7], sy, H[8]);
-      const float* trow = rw.t + dy * rw.tw;
-      const float* wrow = wrow_of(a);
-      const int wst = wst_of(a);
-#pragma unroll 1
-      for (int b = 0; b < wn; ++b) {
-        const int dx = -wr + b * ws;
-        const float sx = fx + (float)dx;
-        const float ik = tile_at(rw, trow + dx);
-        const float w = weight(wrow, wst, b, dx, dy, ik);
-        // the reciprocal is replaced by 0 behind the camera so the discarded fetch coordinates stay finite
-        const float zz = fmaf(H[6], sx, rz);
-        const bool front = zz > 1e-8f;
-        const float izz = front ? m_rcp(zz) : 0.0f;
-        const float sv = sample(fmaf(H[0], sx, rx) * izz, fmaf(H[3], sx, ry) * izz);
-        accumulate(pa, w, front ? sv : 0.0f, ik);
-      }
-    }
-  }
-  return ncc_finish(rs, pair_total<G>(rw, Ss), pair_total<G>(rw, SSs), pair_total<G>(rw, IS));
-}
-
-template <int WR, int WS, bool CW, int NT, bool TEX = false, int G = 1>
-__device__ __forceinline__ float ncc_cost(const PsRun& P, const RefWin& rw, const RefStats& rs, const PsLevel& S,
-                                          const float* H, int x, int y, int& nwin) {
-  if (!ncc_begin(rs, S, H, (float)x, (float)y)) return 2.0f;
-  nwin++;
-  return ncc_window<WR, WS, CW, NT, TEX, G>(P, rw, rs, S, H, x, y);
-}
-
-// ================================================================================ row-pair tap loops (f32x2)
-// The window sums with rows 2p (even) and 2p+1 (odd) in the two halves of f32x2 pairs.  The even-row and odd-row
-// partial sums of the parity contract advance in exactly the order of ncc_window, so the bits are the same, and each
-// pair operation takes one issue slot for two taps.  Sources are sampled by plane loads, a texture gather, or the
-// warp's staged source box (shared memory).
-enum { SMP_LOAD = 0, SMP_TEX = 1, SMP_BOX = 2 };
+// is at one of its four corner taps.  When all four are in front (window_front), every tap is, and the taps run without
+// the per-tap test and selects.
 
 // The warp's staged box: box[r·PS_BOX_P + c] holds texel (gx0 + c, gy0 + r) of the source (0 outside the image);
 // mx = 1.5·2^23 - gx0 and my = 1.5·2^23 - gy0; the taps address it with 32-bit shared-memory addresses.
@@ -477,15 +324,6 @@ struct BoxRef {
   unsigned long long* fault;
 #endif
 };
-// A BoxRef for the samplers that do not read a box (plane loads, texture).
-__device__ __forceinline__ BoxRef no_box(const PsRun& P) {
-  BoxRef b{0u, 0.f, 0.f};
-#if PS_CHECKED
-  b.box = 0u;
-  b.fault = P.fault;
-#endif
-  return b;
-}
 // Checked build: the box texel q (byte address) and its 2 × 2 footprint inside the box.
 __device__ __forceinline__ bool box_in(const BoxRef& bx, unsigned q) {
 #if PS_CHECKED
@@ -525,77 +363,68 @@ __device__ __forceinline__ float lds_off(unsigned a) {
   return v;
 }
 
-template <int SMP>
-__device__ __forceinline__ float2 sample_pair(const PsLevel& S, const BoxRef& bx, float2 u, float2 v) {
-  if constexpr (SMP == SMP_BOX) {
-    const float2 mx = v_splat(bx.mx), my = v_splat(bx.my);
-    const float2 fu = v_add_rm(u, mx), fv = v_add_rm(v, my);
-    const float2 ax = v_sub(u, v_sub(fu, mx));
-    const float2 ay = v_sub(v, v_sub(fv, my));
-    // byte address = base + 4·(bits(Fv)·P + bits(Fu)) with the constant part folded into bx.sbase
-    const unsigned qa = (unsigned)__float_as_int(fv.x) * (4u * PS_BOX_P) + bx.sbase + 4u * (unsigned)__float_as_int(fu.x);
-    const unsigned qb = (unsigned)__float_as_int(fv.y) * (4u * PS_BOX_P) + bx.sbase + 4u * (unsigned)__float_as_int(fu.y);
+__device__ __forceinline__ float2 box_pair(const BoxRef& bx, float2 u, float2 v) {
+  const float2 mx = v_splat(bx.mx), my = v_splat(bx.my);
+  const float2 fu = v_add_rm(u, mx), fv = v_add_rm(v, my);
+  const float2 ax = v_sub(u, v_sub(fu, mx));
+  const float2 ay = v_sub(v, v_sub(fv, my));
+  // byte address = base + 4·(bits(Fv)·P + bits(Fu)) with the constant part folded into bx.sbase
+  const unsigned qa = (unsigned)__float_as_int(fv.x) * (4u * PS_BOX_P) + bx.sbase + 4u * (unsigned)__float_as_int(fu.x);
+  const unsigned qb = (unsigned)__float_as_int(fv.y) * (4u * PS_BOX_P) + bx.sbase + 4u * (unsigned)__float_as_int(fu.y);
 #if PS_CHECKED
-    if (!box_in(bx, qa) || !box_in(bx, qb)) return make_float2(0.f, 0.f);
+  if (!box_in(bx, qa) || !box_in(bx, qb)) return make_float2(0.f, 0.f);
 #endif
-    const float2 p00 = make_float2(lds(qa), lds(qb));
-    const float2 p10 = make_float2(lds_off<4>(qa), lds_off<4>(qb));
-    const float2 p01 = make_float2(lds_off<4 * PS_BOX_P>(qa), lds_off<4 * PS_BOX_P>(qb));
-    const float2 p11 = make_float2(lds_off<4 * PS_BOX_P + 4>(qa), lds_off<4 * PS_BOX_P + 4>(qb));
-    const float2 top = v_fma(ax, v_sub(p10, p00), p00);
-    const float2 bot = v_fma(ax, v_sub(p11, p01), p01);
-    return v_fma(ay, v_sub(bot, top), top);
-  } else if constexpr (SMP == SMP_TEX) {
-    // scalar per lane: the gather's four texels feed the bilinear directly (no repacking into pairs); floorf, not the
-    // FMA-pipe add.rm floor of the box path, which measured 5 % slower here (more registers in the unrolled loop)
-    return make_float2(src_sample_tex(S.tex, u.x, v.x), src_sample_tex(S.tex, u.y, v.y));
-  } else {
-#if PS_CHECKED
-    unsigned long long* const fault = bx.fault;
-#else
-    unsigned long long* const fault = nullptr;
-#endif
-    return make_float2(src_sample(S.img, S.pitch, (float)S.w, (float)S.h, u.x, v.x, fault),
-                       src_sample(S.img, S.pitch, (float)S.w, (float)S.h, u.y, v.y, fault));
-  }
+  const float2 p00 = make_float2(lds(qa), lds(qb));
+  const float2 p10 = make_float2(lds_off<4>(qa), lds_off<4>(qb));
+  const float2 p01 = make_float2(lds_off<4 * PS_BOX_P>(qa), lds_off<4 * PS_BOX_P>(qb));
+  const float2 p11 = make_float2(lds_off<4 * PS_BOX_P + 4>(qa), lds_off<4 * PS_BOX_P + 4>(qb));
+  const float2 top = v_fma(ax, v_sub(p10, p00), p00);
+  const float2 bot = v_fma(ax, v_sub(p11, p01), p01);
+  return v_fma(ay, v_sub(bot, top), top);
 }
 
-template <int SMP>
-__device__ __forceinline__ float sample_one(const PsLevel& S, const BoxRef& bx, float u, float v) {
-  if constexpr (SMP == SMP_BOX) {
-    const float fu = __fadd_rd(u, bx.mx), fv = __fadd_rd(v, bx.my);
-    const float ax = u - (fu - bx.mx), ay = v - (fv - bx.my);
-    const unsigned q = (unsigned)__float_as_int(fv) * (4u * PS_BOX_P) + bx.sbase + 4u * (unsigned)__float_as_int(fu);
-#if PS_CHECKED
-    if (!box_in(bx, q)) return 0.f;
-#endif
-    const float p00 = lds(q), p10 = lds_off<4>(q), p01 = lds_off<4 * PS_BOX_P>(q), p11 = lds_off<4 * PS_BOX_P + 4>(q);
-    const float top = fmaf(ax, p10 - p00, p00);
-    const float bot = fmaf(ax, p11 - p01, p01);
-    return fmaf(ay, bot - top, top);
-  } else if constexpr (SMP == SMP_TEX) {
-    return src_sample_tex(S.tex, u, v);
-  } else {
-#if PS_CHECKED
-    return src_sample(S.img, S.pitch, (float)S.w, (float)S.h, u, v, bx.fault);
-#else
-    return src_sample(S.img, S.pitch, (float)S.w, (float)S.h, u, v);
-#endif
-  }
+// The four corner taps in front of the source camera.
+__device__ __forceinline__ bool window_front(const float* H, float fx, float fy, int wr) {
+  const float sx0 = fx + (float)(-wr), sx1 = fx + (float)wr;
+  const float rz0 = fmaf(H[7], fy + (float)(-wr), H[8]), rz1 = fmaf(H[7], fy + (float)wr, H[8]);
+  return fmaf(H[6], sx0, rz0) > 1e-8f && fmaf(H[6], sx1, rz0) > 1e-8f && fmaf(H[6], sx0, rz1) > 1e-8f &&
+         fmaf(H[6], sx1, rz1) > 1e-8f;
 }
 
-// Window sums of a window whose four corner taps lie in front of the source camera (every tap then does), with the
-// row-pair weight cache.  Rows 2p / 2p+1 go through the pair loop; the last row of an odd window is scalar and adds
-// into the even-row sums, as in ncc_window.  UNROLL unrolls the pair loop over the window columns (the staged path);
-// the rolled form keeps the fallback's code small (instruction-cache footprint of the staged kernel).
-template <int WR, int WS, int NT, int SMP, bool UNROLL>
-__device__ __forceinline__ float ncc_window_pairs(const RefWin& rw, const RefStats& rs, const PsLevel& S, const float* H,
-                                                  int x, int y, const BoxRef& bx) {
-  constexpr int wr = WR, ws = WS, wn = (2 * WR) / WS + 1, np = wn / 2;
+// The cost of a window whose prologue has passed.  The last row of an odd window takes two columns at a time (also a
+// pair) and adds them in column order into the even-row sums.  WR = 0: the window of the parameters, with WS columns
+// unrolled.  ANY: any window (a
+// tap behind the source camera samples 0), else window_front must hold.  BOX: taps from the warp's staged box.
+template <int WR, int WS, bool CW, int NT, bool ANY, bool BOX = false>
+__device__ __forceinline__ float window_sums(const PsRun& P, const RefWin& rw, const RefStats& rs, const PsLevel& S,
+                                             const float* H, int x, int y, const BoxRef& bx = BoxRef()) {
+  const int wr = WR ? WR : P.wr, ws = WR ? WS : P.ws;
+  const int wn = (2 * wr) / ws + 1, np = wn / 2;
+  constexpr int UP = ANY ? 1 : WR ? 2 * WR / WS + 1 : WS, UL = ANY ? 1 : WR ? WR / WS + 1 : WS / 2;
   const float fx = (float)x, fy = (float)y;
+  const unsigned long long tex = S.tex;
   float2 Ss = v_splat(0.f), SSs = v_splat(0.f), IS = v_splat(0.f);
   const float2 h0 = v_splat(H[0]), h1 = v_splat(H[1]), h2 = v_splat(H[2]), h3 = v_splat(H[3]), h4 = v_splat(H[4]),
                h5 = v_splat(H[5]), nh6 = v_splat(-H[6]), nh7 = v_splat(-H[7]), nh8 = v_splat(-H[8]);
+  auto weight = [&](int dx, int dy, float ik) {
+    const float d = rs.ic - ik;
+    return m_exp(-(float)(dx * dx + dy * dy) * P.inv2s - d * d * P.inv2c);
+  };
+  auto sample = [&](float2 nz, float2 un, float2 vn) {
+    if constexpr (ANY) {
+      const bool f0 = -nz.x > 1e-8f, f1 = -nz.y > 1e-8f;
+      const float2 r = m_rcp2(make_float2(f0 ? nz.x : -1.0f, f1 ? nz.y : -1.0f));
+      const float2 izz = make_float2(f0 ? r.x : 0.0f, f1 ? r.y : 0.0f);
+      const float2 u = v_mul(un, izz), v = v_mul(vn, izz);
+      const float2 sv = make_float2(src_sample(tex, u.x, v.x), src_sample(tex, u.y, v.y));
+      return make_float2(f0 ? sv.x : 0.0f, f1 ? sv.y : 0.0f);
+    } else {
+      const float2 izz = m_rcp2(nz);
+      const float2 u = v_mul(un, izz), v = v_mul(vn, izz);
+      if constexpr (BOX) return box_pair(bx, u, v);
+      else return make_float2(src_sample(tex, u.x, v.x), src_sample(tex, u.y, v.y));
+    }
+  };
 #pragma unroll 1
   for (int p = 0; p < np; ++p) {
     const int dy = -wr + 2 * p * ws;
@@ -604,83 +433,60 @@ __device__ __forceinline__ float ncc_window_pairs(const RefWin& rw, const RefSta
     const float* t0 = rw.t + dy * rw.tw;
     const float* t1 = t0 + ws * rw.tw;
     const float* wp = rw.wc + p * wn * NT * 2;
-    auto tap = [&](int dx, float sxf, const float* wq) {
-      const float2 sx = v_splat(sxf);
+#pragma unroll UP
+    for (int b = 0; b < wn; ++b) {
+      const int dx = -wr + b * ws;
+      const float2 sx = v_splat(fx + (float)dx);
       const float2 ik = make_float2(tile_at(rw, t0 + dx), tile_at(rw, t1 + dx));
-      const float2 w = *reinterpret_cast<const float2*>(wq);
-      const float2 izz = m_rcp2(v_fma(nh6, sx, nrz));
-      const float2 sv = sample_pair<SMP>(S, bx, v_mul(v_fma(h0, sx, rx), izz), v_mul(v_fma(h3, sx, ry), izz));
+      float2 w;
+      if constexpr (CW) w = *reinterpret_cast<const float2*>(wp + b * NT * 2);
+      else w = make_float2(weight(dx, dy, ik.x), weight(dx, dy + ws, ik.y));
+      const float2 sv = sample(v_fma(nh6, sx, nrz), v_fma(h0, sx, rx), v_fma(h3, sx, ry));
       const float2 wsv = v_mul(w, sv);
       Ss = v_add(Ss, wsv);
       SSs = v_fma(wsv, sv, SSs);
       IS = v_fma(wsv, ik, IS);
-    };
-    if constexpr (UNROLL) {
-#pragma unroll
-      for (int b = 0; b < wn; ++b) tap(-wr + b * ws, fx + (float)(-wr + b * ws), wp + b * NT * 2);
-    } else {
-      int dx = -wr;
-      float sxf = fx + (float)(-wr);
-      const float* wq = wp;
-#pragma unroll 1
-      for (int b = 0; b < wn; ++b) {
-        tap(dx, sxf, wq);
-        dx += ws;
-        sxf += (float)ws;
-        wq += NT * 2;
-      }
     }
   }
-  if constexpr ((wn & 1) != 0) {
+  if ((wn & 1) != 0) {
     const int dy = -wr + (wn - 1) * ws;
     const float sy = fy + (float)dy;
-    const float rx = fmaf(H[1], sy, H[2]), ry = fmaf(H[4], sy, H[5]), rz = fmaf(H[7], sy, H[8]);
+    const float2 rx = v_splat(fmaf(H[1], sy, H[2])), ry = v_splat(fmaf(H[4], sy, H[5]));
+    const float2 nrz = v_splat(-fmaf(H[7], sy, H[8]));
     const float* t0 = rw.t + dy * rw.tw;
-    auto tap = [&](int b, int dx, float sx) {
-      const float ik = tile_at(rw, t0 + dx);
-      const float w = rw.wl[b * NT];
-      const float izz = m_rcp(fmaf(H[6], sx, rz));
-      const float sv = sample_one<SMP>(S, bx, fmaf(H[0], sx, rx) * izz, fmaf(H[3], sx, ry) * izz);
-      const float wsv = w * sv;
-      Ss.x = Ss.x + wsv;
-      SSs.x = fmaf(wsv, sv, SSs.x);
-      IS.x = fmaf(wsv, ik, IS.x);
-    };
-    if constexpr (UNROLL) {
-#pragma unroll
-      for (int b = 0; b < wn; ++b) tap(b, -wr + b * ws, fx + (float)(-wr + b * ws));
-    } else {
-      int dx = -wr;
-      float sx = fx + (float)(-wr);
-#pragma unroll 1
-      for (int b = 0; b < wn; ++b) {
-        tap(b, dx, sx);
-        dx += ws;
-        sx += (float)ws;
+#pragma unroll UL
+    for (int b = 0; b < wn; b += 2) {
+      const int b1 = min(b + 1, wn - 1);  // the last column stands alone; its second half is not added
+      const int dx = -wr + b * ws, dx1 = -wr + b1 * ws;
+      const float2 sx = make_float2(fx + (float)dx, fx + (float)dx1);
+      const float2 ik = make_float2(tile_at(rw, t0 + dx), tile_at(rw, t0 + dx1));
+      float2 w;
+      if constexpr (CW) w = make_float2(rw.wl[b * NT], rw.wl[b1 * NT]);
+      else w = make_float2(weight(dx, dy, ik.x), weight(dx1, dy, ik.y));
+      const float2 sv = sample(v_fma(nh6, sx, nrz), v_fma(h0, sx, rx), v_fma(h3, sx, ry));
+      const float2 wsv = v_mul(w, sv);
+      Ss.x = Ss.x + wsv.x;
+      SSs.x = fmaf(wsv.x, sv.x, SSs.x);
+      IS.x = fmaf(wsv.x, ik.x, IS.x);
+      if (b1 != b) {
+        Ss.x = Ss.x + wsv.y;
+        SSs.x = fmaf(wsv.y, sv.y, SSs.x);
+        IS.x = fmaf(wsv.y, ik.y, IS.x);
       }
     }
   }
   return ncc_finish(rs, Ss.x + Ss.y, SSs.x + SSs.y, IS.x + IS.y);
 }
 
-// Corner test of ncc_window: the four corner taps in front of the source camera.
-template <int WR>
-__device__ __forceinline__ bool window_front(const float* H, float fx, float fy) {
-  const float sx0 = fx + (float)(-WR), sx1 = fx + (float)WR;
-  const float rz0 = fmaf(H[7], fy + (float)(-WR), H[8]), rz1 = fmaf(H[7], fy + (float)WR, H[8]);
-  return fmaf(H[6], sx0, rz0) > 1e-8f && fmaf(H[6], sx1, rz0) > 1e-8f && fmaf(H[6], sx0, rz1) > 1e-8f &&
-         fmaf(H[6], sx1, rz1) > 1e-8f;
-}
-
-// One lane's window with the row-pair loops (the prologue must have passed): pair loop when the window is wholly in
-// front, otherwise the guarded loop of ncc_window on the row-pair cache.
-template <int WR, int WS, int NT, bool TEX>
-__device__ __forceinline__ float ncc_window_lane(const PsRun& P, const RefWin& rw, const RefStats& rs,
-                                                 const PsLevel& S, const float* H, int x, int y) {
-  constexpr int smp = TEX ? SMP_TEX : SMP_LOAD;
-  if (window_front<WR>(H, (float)x, (float)y))
-    return ncc_window_pairs<WR, WS, NT, smp, true>(rw, rs, S, H, x, y, no_box(P));
-  return ncc_window<WR, WS, true, NT, TEX, 1, true>(P, rw, rs, S, H, x, y);
+// Cost of one window (patchmatch.cu:245-290) through texture gathers, with the weight cache (CW) or recomputed weights.
+template <int WR, int WS, bool CW, int NT>
+__device__ __forceinline__ float ncc_cost(const PsRun& P, const RefWin& rw, const RefStats& rs, const PsLevel& S,
+                                             const float* H, int x, int y, int& nwin) {
+  if (!ncc_begin(rs, S, H, (float)x, (float)y)) return 2.0f;
+  nwin++;
+  if (window_front(H, (float)x, (float)y, WR ? WR : P.wr))
+    return window_sums<WR, WS, CW, NT, false>(P, rw, rs, S, H, x, y);
+  return window_sums<WR, WS, CW, NT, true>(P, rw, rs, S, H, x, y);
 }
 
 // ------------------------------------------------------------------------------------------- TMA staging
@@ -751,7 +557,7 @@ struct BoxState {
 // a restage centres the box on the request and copies it with 16-byte cp.async chunks.  Windows that fail the bound,
 // a request wider than PS_BOX_P - 3 or taller than PS_BOX_H texels, or fewer than PS_STAGE_MIN_LANES active lanes use
 // the per-lane loops.  All paths give the same bits.
-template <int WR, int WS, int NT, bool TEX, bool TMA>
+template <int WR, int WS, int NT, bool TMA>
 __device__ __forceinline__ float ncc_cost_warp(const PsRun& P, const RefWin& rw, const RefStats& rs, const PsLevel& S,
                                                int src, const float* H, int x, int y, bool act, int& nwin, float* box,
                                                BoxState& bs) {
@@ -855,13 +661,12 @@ __device__ __forceinline__ float ncc_cost_warp(const PsRun& P, const RefWin& rw,
       bx.box = (unsigned)__cvta_generic_to_shared(box);
       bx.fault = P.fault;
 #endif
-      return act ? ncc_window_pairs<WR, WS, NT, SMP_BOX, true>(rw, rs, S, H, x, y, bx) : 2.0f;
+      return act ? window_sums<WR, WS, true, NT, false, true>(P, rw, rs, S, H, x, y, bx) : 2.0f;
     }
   }
   if (!act) return 2.0f;
-  if (front)
-    return ncc_window_pairs<WR, WS, NT, TEX ? SMP_TEX : SMP_LOAD, true>(rw, rs, S, H, x, y, no_box(P));
-  return ncc_window<WR, WS, true, NT, TEX, 1, true>(P, rw, rs, S, H, x, y);
+  if (front) return window_sums<WR, WS, true, NT, false>(P, rw, rs, S, H, x, y);
+  return window_sums<WR, WS, true, NT, true>(P, rw, rs, S, H, x, y);
 }
 
 // Forward/backward reprojection error through the source snapshot (patchmatch.cu:292-314); INF on failure.
@@ -892,13 +697,13 @@ __device__ float geo_error(const PsRun& P, const PsLevel& R, const PsLevel& S, c
 }
 
 // (photometric cost, truncated geometric error) of one hypothesis × one source (patchmatch.cu:316-324).
-template <int WR, int WS, bool CW, int NT, bool TEX = false, int G = 1>
+template <int WR, int WS, bool CW, int NT>
 __device__ __forceinline__ float pair_cost(const PsRun& P, const RefWin& rw, const RefStats& rs, const PsLevel& R,
                                            const PsLevel& S, const PsPair& pr, const PsLPair& lp, int x, int y,
                                            float4 h, float* geo, int& nwin) {
   float H[9];
   float c = 2.0f;
-  if (homography(R, lp, (float)x, (float)y, h, H)) c = ncc_cost<WR, WS, CW, NT, TEX, G>(P, rw, rs, S, H, x, y, nwin);
+  if (homography(R, lp, (float)x, (float)y, h, H)) c = ncc_cost<WR, WS, CW, NT>(P, rw, rs, S, H, x, y, nwin);
   if (P.geometric) *geo = fminf(geo_error(P, R, S, pr, x, y, h.w), P.gmax);
   return c;
 }
@@ -1031,15 +836,10 @@ __device__ __forceinline__ void count_skipped(const PsRun& P, int n) {
   if ((int)(threadIdx.x & 31) == __ffs(m) - 1 && s) atomicAdd(P.stage_count + 6, (unsigned long long)s);
 }
 
-// Half-step tile geometry for G lanes per pixel: G = 1 -> 32 × 8 pixels (a warp = 16 active columns × 2 rows);
-// G = 2 -> 16 × 8 pixels (a warp = 8 active columns × 2 rows × 2 lanes).  The shared tile's row pitch is padded so
-// that the lanes of one warp read 32 distinct banks: even for G = 1, ≡ 16 (mod 32) for G = 2.  The staged kernel's
-// warp (4 active columns × 8 rows) needs a pitch ≡ 4 or 12 (mod 16): its same-parity rows then fall 8 banks apart
-// and the checkerboard puts the other rows on the other bank parity.
-__host__ __device__ constexpr int half_pw(int G) { return G == 2 ? PS_HALF2_PW : PS_HALF_PW; }
-__host__ __device__ constexpr int half_tw(int G, int wr) {
-  return G == 2 ? (((PS_HALF2_PW + 2 * wr) + 15) / 32) * 32 + 16 : PS_HALF_PW + 2 * wr;
-}
+// Half-step tile: 32 × 8 pixels, a warp = 16 active columns × 2 rows.  The staged kernel's warp (4 active columns × 8 rows)
+// needs a tile pitch ≡ 4 or 12 (mod 16): its same-parity rows then fall 8 banks apart and the checkerboard puts the other
+// rows on the other bank parity.
+__host__ __device__ constexpr int half_tw(int wr) { return PS_HALF_PW + 2 * wr; }
 __host__ __device__ constexpr int half_tw_staged(int wr) { return PS_HALF_ST_TW(wr); }
 
 // ---------------------------------------------------------------------------- per-pixel PatchMatch logic
@@ -1218,33 +1018,33 @@ __device__ __forceinline__ float4 refine_candidate(const Refine& r, int c) {
   }
 }
 
-// Half-step variants (all give the same bits):
-//   k_half MODE 0: one lane (G = 1) or two lanes (G = 2) per pixel, scalar tap loops;
-//   k_half MODE 1: one lane per pixel, row-pair f32x2 tap loops on the row-pair weight cache;
-//   k_half_st:     row pairs plus the warp-collective staged source boxes (ncc_cost_warp).
-// G = 1: two CTAs per SM with the weight cache (~90 KB each for a 13×13 window), four without it.
-// G = 2: the two lanes of a pixel split the window rows, so each thread caches half the weights: four CTAs per SM.
+// CTAs per SM that the half step's registers are sized for.  A gather answers after many hundred cycles, so what counts
+// is how many a CTA keeps in flight: the whole column loop is unrolled (26 gathers at 13 columns; unrolled by 4 the same
+// kernel takes 2.6 times as long), and that takes about 250 registers.  Two CTAs fill the register file then, and for the
+// windows of 11 and 13 columns their weight caches fill the shared memory as well.  Windows of up to 7 columns have few
+// gathers per row and a small cache: four CTAs with 128 registers hide more (4 views of 640 × 480 and 4 sources, ms per
+// half step with two and four: 1.98 -> 1.85 at 11×11 step 2, 2.58 -> 2.39 at 7×7).
+__host__ __device__ constexpr int half_min_ctas(int wr, int ws) {
+  return wr == 0 ? (ws == 4 ? 4 : 2) : 2 * wr / ws + 1 <= 7 ? 4 : 2;
+}
 // One half-step tile: CTA `cta` of the launch's flattened tile list, in phase `ph`, with dynamic shared memory sm.
-template <int WR, int WS, bool CW, bool TEX, int G, int MODE>
+template <int WR, int WS, bool CW>
 __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, int cta, float* sm) {
   constexpr int NT = PS_HALF_NT;
-  constexpr int PW = half_pw(G);
-  constexpr bool PAIRW = MODE >= 1;
-  static_assert(MODE == 0 || (MODE == 1 && CW && G == 1 && WR != 0), "row pairs need the weight cache, one lane, a fixed window");
   const int wr = WR ? WR : P.wr, ws = WR ? WS : P.ws;
   const int wn = (2 * wr) / ws + 1;
-  const int TW = half_tw(G, wr), TH = PS_HALF_PH + 2 * wr;
+  const int TW = half_tw(wr), TH = PS_HALF_PH + 2 * wr;
   float* tile = sm;
   float* wcache = sm + ((TW * TH + 31) & ~31);
-  float* wvs = wcache + (CW ? ((wn + G - 1) / G) * wn * NT : 0);
+  float* wvs = wcache + (CW ? wn * wn * NT : 0);
 
   const int ii = find_item(P, cta);
   const PsItem& it = P.items[ii];
   if (!item_ok(P, it)) return;
   const int w = it.w, h = it.h;
-  const int tiles_x = (w + PW - 1) / PW;
+  const int tiles_x = (w + PS_HALF_PW - 1) / PS_HALF_PW;
   const int tl = cta - it.tile0;
-  const int x0 = (tl % tiles_x) * PW, y0 = (tl / tiles_x) * PS_HALF_PH;
+  const int x0 = (tl % tiles_x) * PS_HALF_PW, y0 = (tl / tiles_x) * PS_HALF_PH;
   const PsLevel R = P.lv[it.view * P.nlevels + P.level];
   {
     const int ox = x0 - wr, oy = y0 - wr;
@@ -1256,20 +1056,16 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int gl = G == 2 ? (lane & 1) : 0;
-  const int row = 2 * warp + (lane >> 4), col = G == 2 ? ((lane >> 1) & 7) : (lane & 15);
+  const int row = 2 * warp + (lane >> 4), col = lane & 15;
   const int y = y0 + row;
   const int x = x0 + 2 * col + ((y + ph.color) & 1);
-  if (x >= w || y >= h) return;  // both lanes of a pixel leave together
+  if (x >= w || y >= h) return;
 
   RefWin rw;
   rw.t = tile + (row + wr) * TW + (x - x0 + wr);
   rw.tw = TW;
   refwin_bounds(rw, tile, TW * TH, P);
-  rw.wc = wcache + (PAIRW ? 2 * threadIdx.x : threadIdx.x);
-  rw.g = gl;
-  rw.pmask = G == 2 ? (3u << (lane & ~1)) : 0u;
-  rw.wl = wcache + (wn & ~1) * wn * NT + threadIdx.x;
+  refwin_cache<NT>(rw, wcache, wn);
   float* wv = wvs + threadIdx.x;
 
   const PsView& vd = P.views[it.view];
@@ -1286,15 +1082,9 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
 
   // One NCC window of this pixel (the homography H is valid where hok).
   int nwin = 0;
-  const RefStats rs = ref_stats<WR, WS, CW, NT, G, PAIRW>(P, rw);
+  const RefStats rs = ref_stats<WR, WS, CW, NT>(P, rw);
   auto window = [&](const PsLevel& S, const float* H, bool hok) -> float {
-    if constexpr (MODE == 1) {
-      if (!hok || !ncc_begin(rs, S, H, (float)x, (float)y)) return 2.0f;
-      nwin++;
-      return ncc_window_lane<WR, WS, NT, TEX>(P, rw, rs, S, H, x, y);
-    } else {
-      return hok ? ncc_cost<WR, WS, CW, NT, TEX, G>(P, rw, rs, S, H, x, y, nwin) : 2.0f;
-    }
+    return hok ? ncc_cost<WR, WS, CW, NT>(P, rw, rs, S, H, x, y, nwin) : 2.0f;
   };
 
   // 2. View traversal: voting, weighting, aggregation.
@@ -1377,19 +1167,17 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
       best = cd;
     }
   }
-  if (gl == 0) {
-    pl[pix] = best;
-    P.cost[base + pix] = bcost;
-    P.bview[base + pix] = (unsigned char)ag.vbest;
-  }
-  count_windows(P, gl == 0 ? nwin : 0);
-  count_skipped(P, gl == 0 ? nskip : 0);
+  pl[pix] = best;
+  P.cost[base + pix] = bcost;
+  P.bview[base + pix] = (unsigned char)ag.vbest;
+  count_windows(P, nwin);
+  count_skipped(P, nskip);
 }
 
-template <int WR, int WS, bool CW, bool TEX, int G, int MODE = 0>
-__global__ void __launch_bounds__(PS_HALF_NT, (CW && G == 1) ? 2 : 4) k_half(const __grid_constant__ PsRun P) {
+template <int WR, int WS, bool CW>
+__global__ void __launch_bounds__(PS_HALF_NT, half_min_ctas(WR, WS)) k_half(const __grid_constant__ PsRun P) {
   extern __shared__ float sm[];
-  half_tile<WR, WS, CW, TEX, G, MODE>(P, launch_phase(P), blockIdx.x, sm);
+  half_tile<WR, WS, CW>(P, launch_phase(P), blockIdx.x, sm);
 }
 
 // ================================================================================ persistent half step (PS_TUNE_PERSISTENT)
@@ -1423,8 +1211,8 @@ __device__ __forceinline__ bool queue_wait(const PsRun& P, const unsigned* ctr, 
 // A CTA that has seen phase k - 1 of a view complete (an acquire) needs no second wait for it: its later loads see
 // those stores.  It remembers the last completed phase per view (s_seen), so a CTA waits about once per view and
 // phase instead of once per tile.
-template <int WR, int WS, bool TEX>
-__global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_q(const __grid_constant__ PsRun P) {
+template <int WR, int WS>
+__global__ void __launch_bounds__(PS_HALF_NT, half_min_ctas(WR, WS)) k_half_q(const __grid_constant__ PsRun P) {
   extern __shared__ float sm[];
   __shared__ int s_item, s_go;
   __shared__ int s_seen[PS_MAX_ITEMS];
@@ -1456,7 +1244,7 @@ __global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_q(const __grid_constant_
     const int k = i / P.ntiles, cta = i - k * P.ntiles;
     if (s_go) {
       const PsPhase& q = P.phases[k];
-      half_tile<WR, WS, true, TEX, 1, 1>(P, HalfPhase{q.t, q.color, q.tau_good, q.eps, q.phi}, cta, sm);
+      half_tile<WR, WS, true>(P, HalfPhase{q.t, q.color, q.tau_good, q.eps, q.phi}, cta, sm);
     }
     __syncthreads();  // the tile's stores (and its reads of s_item) are done
     if (threadIdx.x == 0) {
@@ -1478,7 +1266,7 @@ __global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_q(const __grid_constant_
 // column (so its first element is 16-byte aligned) and reads the plane's zero border, padding and out-of-tensor zeros
 // where the copy loop writes zeros outside the image: the same values.
 __host__ __device__ constexpr int tma_xo(int wr) { return wr + ((PS_BORDER - wr) & 3); }
-template <int WR, int WS, bool TEX, bool TMA>
+template <int WR, int WS, bool TMA>
 __global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_st(const __grid_constant__ PsRun P) {
   constexpr int NT = PS_HALF_NT;
   constexpr int wr = WR, wn = (2 * WR) / WS + 1;
@@ -1541,10 +1329,7 @@ __global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_st(const __grid_constant
   rw.t = tile + (y - y0 + wr) * TW + (x - x0 + XO);
   rw.tw = TW;
   refwin_bounds(rw, tile, TW * TH, P);
-  rw.wc = wcache + 2 * threadIdx.x;
-  rw.g = 0;
-  rw.pmask = 0u;
-  rw.wl = wcache + (wn & ~1) * wn * NT + threadIdx.x;
+  refwin_cache<NT>(rw, wcache, wn);
   float* wv = wvs + threadIdx.x;
 
   const PsView& vd = P.views[it.view];
@@ -1560,7 +1345,7 @@ __global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_st(const __grid_constant
   float4 hyp[9];
   propagation_candidates(R, pl, P.cost + base, x, y, w, h, ray, hyp);
   int nwin = 0;
-  const RefStats rs = ref_stats<WR, WS, true, NT, 1, true>(P, rw);
+  const RefStats rs = ref_stats<WR, WS, true, NT>(P, rw);
   const int vprev = P.bview[base + pix];
   Refine rf;
   refine_prior(P, base + pix, rs.var, ray, rf);
@@ -1621,7 +1406,7 @@ __global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_st(const __grid_constant
     if (__any_sync(FULL, act)) {
       float H[9];
       const bool hok = homography(R, lp, fx, fy, hv, H);
-      mv = ncc_cost_warp<WR, WS, NT, TEX, TMA>(P, rw, rs, S, pr.src, H, x, y, act && hok, nwin, box, bs);
+      mv = ncc_cost_warp<WR, WS, NT, TMA>(P, rw, rs, S, pr.src, H, x, y, act && hok, nwin, box, bs);
     }
     if (trav) {
       const float gv = (P.geometric && use) ? fminf(geo_error(P, R, S, pr, x, y, hv.w), P.gmax) : 0.f;
@@ -1671,7 +1456,7 @@ __global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_st(const __grid_constant
 
 // ================================================================================ run start / evaluate (patchmatch.cu:661-692)
 // Top-K mean cost (patchmatch.cu:327-345).
-template <int WR, int WS, bool CW, int NT, bool TEX = false>
+template <int WR, int WS, bool CW, int NT>
 __device__ float topk_cost(const PsRun& P, const RefWin& rw, const RefStats& rs, const PsLevel& R, const PsPair* prs,
                            const PsLPair* lps, int nsrc, int x, int y, float4 h, int& nwin) {
   float b0 = 1e30f, b1 = 1e30f, b2 = 1e30f;
@@ -1681,7 +1466,7 @@ __device__ float topk_cost(const PsRun& P, const RefWin& rw, const RefStats& rs,
     const PsLPair lp = lps[j];
     const PsLevel S = P.lv[pr.src * P.nlevels + P.level];
     float g = 0.f;
-    float c = pair_cost<WR, WS, CW, NT, TEX>(P, rw, rs, R, S, pr, lp, x, y, h, &g, nwin);
+    float c = pair_cost<WR, WS, CW, NT>(P, rw, rs, R, S, pr, lp, x, y, h, &g, nwin);
     if (P.geometric) c += P.lambda * g;
     if (c < b0) {
       b2 = b1;
@@ -1731,9 +1516,8 @@ __device__ __forceinline__ bool eval_tile(const PsRun& P, float* tile, int wr, E
   return e.x < it.w && e.y < it.h;
 }
 
-// TEX: the source samples through the planes' texture gathers (same bits as the plane loads).
-template <int WR, int WS, bool CW, bool TEX>
-__global__ void __launch_bounds__(PS_EVAL_NT, 2) k_eval(const __grid_constant__ PsRun P) {
+template <int WR, int WS, bool CW>
+__global__ void __launch_bounds__(PS_EVAL_NT, half_min_ctas(WR, WS)) k_eval(const __grid_constant__ PsRun P) {
   constexpr int NT = PS_EVAL_NT;
   extern __shared__ float sm[];
   const int wr = WR ? WR : P.wr;
@@ -1750,7 +1534,7 @@ __global__ void __launch_bounds__(PS_EVAL_NT, 2) k_eval(const __grid_constant__ 
   }
   rw.tw = TW;
   refwin_bounds(rw, sm, TW * TH, P);
-  rw.wc = sm + ((TW * TH + 31) & ~31) + threadIdx.x;
+  refwin_cache<NT>(rw, sm + ((TW * TH + 31) & ~31), (2 * wr) / (WR ? WS : P.ws) + 1);
   const PsItem& it = *e.it;
   const PsView& vd = P.views[it.view];
   const PsPair* prs = P.pairs + (size_t)it.view * PS_MAXSRC;
@@ -1774,7 +1558,7 @@ __global__ void __launch_bounds__(PS_EVAL_NT, 2) k_eval(const __grid_constant__ 
   int nwin = 0;
   if (h.w > 0.f) {
     const RefStats rs = ref_stats<WR, WS, CW, NT>(P, rw);
-    c = topk_cost<WR, WS, CW, NT, TEX>(P, rw, rs, e.R, prs, lps, vd.nsrc, x, y, h, nwin);
+    c = topk_cost<WR, WS, CW, NT>(P, rw, rs, e.R, prs, lps, vd.nsrc, x, y, h, nwin);
   }
   P.cost[base + pix] = c;
   if (P.mode == 1) P.bview[base + pix] = 255;
@@ -1793,8 +1577,8 @@ __device__ __forceinline__ unsigned short bf16_bits(float v) {
   return *reinterpret_cast<const unsigned short*>(&b);
 }
 
-template <int WR, int WS, bool TEX>
-__global__ void __launch_bounds__(PS_EVAL_NT, 2) k_sweep(const __grid_constant__ PsRun P) {
+template <int WR, int WS>
+__global__ void __launch_bounds__(PS_EVAL_NT, half_min_ctas(WR, WS)) k_sweep(const __grid_constant__ PsRun P) {
   constexpr int NT = PS_EVAL_NT;
   extern __shared__ float sm[];
   const int wr = WR ? WR : P.wr;
@@ -1811,7 +1595,7 @@ __global__ void __launch_bounds__(PS_EVAL_NT, 2) k_sweep(const __grid_constant__
   }
   rw.tw = TW;
   refwin_bounds(rw, sm, TW * TH, P);
-  rw.wc = sm + ((TW * TH + 31) & ~31) + threadIdx.x;
+  refwin_cache<NT>(rw, sm + ((TW * TH + 31) & ~31), (2 * wr) / (WR ? WS : P.ws) + 1);
   const PsView& vd = P.views[e.it->view];
   const PsLPair* lps = P.lpairs + ((size_t)e.it->view * P.nlevels + P.level) * PS_MAXSRC;
   const PsPair* prs = P.pairs + (size_t)e.it->view * PS_MAXSRC;
@@ -1831,7 +1615,7 @@ __global__ void __launch_bounds__(PS_EVAL_NT, 2) k_sweep(const __grid_constant__
       const PsLevel S = P.lv[prs[j].src * P.nlevels + P.level];
       float H[9];
       c += homography(e.R, lps[j], (float)x, (float)y, h, H)
-               ? ncc_cost<WR, WS, true, NT, TEX>(P, rw, rs, S, H, x, y, nwin)
+               ? ncc_cost<WR, WS, true, NT>(P, rw, rs, S, H, x, y, nwin)
                : 2.0f;
     }
     c = nuse == 2 ? c * 0.5f : (nuse == 1 ? c : 2.0f);
@@ -1843,8 +1627,8 @@ __global__ void __launch_bounds__(PS_EVAL_NT, 2) k_sweep(const __grid_constant__
 }
 
 // ================================================================================ final readout (patchmatch.cu:695-737)
-template <int WR, int WS, bool CW, bool TEX>
-__global__ void __launch_bounds__(PS_EVAL_NT, 2) k_filter(const __grid_constant__ PsRun P) {
+template <int WR, int WS, bool CW>
+__global__ void __launch_bounds__(PS_EVAL_NT, half_min_ctas(WR, WS)) k_filter(const __grid_constant__ PsRun P) {
   constexpr int NT = PS_EVAL_NT;
   extern __shared__ float sm[];
   const int wr = WR ? WR : P.wr;
@@ -1862,7 +1646,7 @@ __global__ void __launch_bounds__(PS_EVAL_NT, 2) k_filter(const __grid_constant_
   }
   rw.tw = TW;
   refwin_bounds(rw, sm, TW * TH, P);
-  rw.wc = sm + ((TW * TH + 31) & ~31) + threadIdx.x;
+  refwin_cache<NT>(rw, sm + ((TW * TH + 31) & ~31), (2 * wr) / (WR ? WS : P.ws) + 1);
   const PsView& vd = P.views[it.view];
   const PsPair* prs = P.pairs + (size_t)it.view * PS_MAXSRC;
   const PsLPair* lps = P.lpairs + ((size_t)it.view * P.nlevels + P.level) * PS_MAXSRC;
@@ -1890,7 +1674,7 @@ __global__ void __launch_bounds__(PS_EVAL_NT, 2) k_filter(const __grid_constant_
       float H[9];
       const PsLPair lp = lps[j];
       if (!homography(e.R, lp, (float)x, (float)y, h, H)) continue;
-      const float m = ncc_cost<WR, WS, CW, NT, TEX>(P, rw, rs, S, H, x, y, nwin);
+      const float m = ncc_cost<WR, WS, CW, NT>(P, rw, rs, S, H, x, y, nwin);
       const float ee = P.ncc_norm * m_exp(-m * m * P.inv2ncc);
       if (ee / (ee + 0.5f) < P.q_min) continue;
       if (geo_error(P, e.R, S, pr, x, y, h.w) > P.filter_gmax) continue;
@@ -2155,11 +1939,11 @@ static cudaError_t init_constants() {
   return e;
 }
 
-size_t half_smem(int wr, int ws, bool cw, int maxsrc, int G, int mode) {
+size_t half_smem(int wr, int ws, bool cw, int maxsrc, bool staged) {
   const int wn = (2 * wr) / ws + 1;
-  const int TW = mode == 2 ? half_tw_staged(wr) : half_tw(G, wr), TH = PS_HALF_PH + 2 * wr;
-  size_t f = ((TW * TH + 31) & ~31) + (cw ? (size_t)((wn + G - 1) / G) * wn * PS_HALF_NT : 0) +
-             (size_t)maxsrc * PS_HALF_NT + (mode == 2 ? (size_t)(PS_HALF_NT / 32) * PS_BOX_P * PS_BOX_H : 0);
+  const int TW = staged ? half_tw_staged(wr) : half_tw(wr), TH = PS_HALF_PH + 2 * wr;
+  size_t f = ((TW * TH + 31) & ~31) + (cw ? (size_t)wn * wn * PS_HALF_NT : 0) + (size_t)maxsrc * PS_HALF_NT +
+             (staged ? (size_t)(PS_HALF_NT / 32) * PS_BOX_P * PS_BOX_H : 0);
   return f * sizeof(float);
 }
 size_t eval_smem(int wr, int ws, bool cw) {
@@ -2170,7 +1954,7 @@ size_t eval_smem(int wr, int ws, bool cw) {
 }
 
 // Whether the weight cache fits (<= 200 KB of shared memory per CTA with the largest source count).
-static bool use_cache(int wr, int ws) { return half_smem(wr, ws, true, PS_MAXSRC, 1, 0) <= 200 * 1024; }
+static bool use_cache(int wr, int ws) { return half_smem(wr, ws, true, PS_MAXSRC, false) <= 200 * 1024; }
 
 template <typename K>
 static cudaError_t launch(K kern, int ncta, int nt, size_t smem, cudaStream_t st, const PsRun& P) {
@@ -2182,49 +1966,29 @@ static cudaError_t launch(K kern, int ncta, int nt, size_t smem, cudaStream_t st
   return cudaGetLastError();
 }
 
-// Half-step mode of a tuning word: 2 = staged source boxes (PS_TUNE_STAGED), 1 = row-pair loops (PS_TUNE_ROW_PAIRS),
-// 0 = scalar loops.  The row-pair modes need one lane per pixel, the weight cache and a compiled window; otherwise the
-// scalar kernel runs (same bits).
-static int half_mode(unsigned tuning, int wr, int ws) {
-  if (!(tuning & 0x18u) || (tuning & 0x1u) || !use_cache(wr, ws)) return 0;
+// Whether (wr, ws) has kernels of its own.
+static bool compiled_window(int wr, int ws) {
   bool compiled = false;
 #define PS_CASE(a, b) compiled = compiled || (wr == a && ws == b);
   PS_SPECS(PS_CASE)
 #undef PS_CASE
-  if (!compiled) return 0;
-  return (tuning & 0x10u) ? 2 : 1;
+  return compiled;
+}
+// Whether the half step stages source boxes: PS_TUNE_STAGED at a compiled window.
+static bool half_staged(unsigned tuning, int wr, int ws) {
+  return (tuning & 0x10u) && !(tuning & 0x1u) && compiled_window(wr, ws);
 }
 
-// Lanes per pixel of the half-step kernel for a tuning word (PS_TUNE_ONE_LANE or a row-pair mode selects 1, default 2).
-int half_lanes(unsigned tuning) { return (tuning & 0x1Cu) ? 1 : 2; }
-
-template <int A, int B, int G>
-static cudaError_t launch_half_g(const PsRun& P, bool cw, bool tex, size_t smem, cudaStream_t st) {
-  if (cw) return tex ? launch(k_half<A, B, true, true, G>, P.ntiles, PS_HALF_NT, smem, st, P)
-                     : launch(k_half<A, B, true, false, G>, P.ntiles, PS_HALF_NT, smem, st, P);
-  return tex ? launch(k_half<A, B, false, true, G>, P.ntiles, PS_HALF_NT, smem, st, P)
-             : launch(k_half<A, B, false, false, G>, P.ntiles, PS_HALF_NT, smem, st, P);
+// Whether the persistent kernel runs a run's half steps for this tuning word and window: PS_TUNE_PERSISTENT with
+// PS_TUNE_ROW_PAIRS at a compiled window.
+bool half_run_ok(unsigned tuning, int wr, int ws) {
+  return (tuning & 0x28u) == 0x28u && !(tuning & 0x11u) && compiled_window(wr, ws);
 }
-template <int A, int B>
-static cudaError_t launch_half_pairs(const PsRun& P, int mode, bool tex, size_t smem, cudaStream_t st) {
-  if (mode == 2) {
-    if (P.tmaps) return tex ? launch(k_half_st<A, B, true, true>, P.ntiles, PS_HALF_NT, smem, st, P)
-                            : launch(k_half_st<A, B, false, true>, P.ntiles, PS_HALF_NT, smem, st, P);
-    return tex ? launch(k_half_st<A, B, true, false>, P.ntiles, PS_HALF_NT, smem, st, P)
-               : launch(k_half_st<A, B, false, false>, P.ntiles, PS_HALF_NT, smem, st, P);
-  }
-  return tex ? launch(k_half<A, B, true, true, 1, 1>, P.ntiles, PS_HALF_NT, smem, st, P)
-             : launch(k_half<A, B, true, false, 1, 1>, P.ntiles, PS_HALF_NT, smem, st, P);
-}
-
-// Whether the persistent kernel runs a run's half steps for this tuning word and window: the row-pair mode with
-// PS_TUNE_PERSISTENT.
-bool half_run_ok(unsigned tuning, int wr, int ws) { return (tuning & 0x20u) && half_mode(tuning, wr, ws) == 1; }
 
 // The persistent half step: as many CTAs as fit on the device at once (or fewer when there are fewer items).
 template <int A, int B>
-static cudaError_t launch_half_q(const PsRun& P, bool tex, size_t smem, cudaStream_t st) {
-  void (*kern)(PsRun) = tex ? k_half_q<A, B, true> : k_half_q<A, B, false>;
+static cudaError_t launch_half_q(const PsRun& P, size_t smem, cudaStream_t st) {
+  void (*kern)(PsRun) = k_half_q<A, B>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int dev = 0, sms = 0, per = 0;
@@ -2244,10 +2008,9 @@ cudaError_t launch_half_run(const PsRun& P, unsigned tuning, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   if (!half_run_ok(tuning, P.wr, P.ws) || !P.queue || P.nphases < 1 || P.nphases > PS_MAX_PHASES)
     return cudaErrorInvalidValue;
-  const bool tex = (tuning & 0x2u) != 0;
-  const size_t smem = half_smem(P.wr, P.ws, true, P.maxsrc, 1, 1);
+  const size_t smem = half_smem(P.wr, P.ws, true, P.maxsrc, false);
 #define PS_CASE(a, b) \
-  if (P.wr == a && P.ws == b) return launch_half_q<a, b>(P, tex, smem, st);
+  if (P.wr == a && P.ws == b) return launch_half_q<a, b>(P, smem, st);
   PS_SPECS(PS_CASE)
 #undef PS_CASE
   return cudaErrorInvalidValue;
@@ -2256,54 +2019,50 @@ cudaError_t launch_half_run(const PsRun& P, unsigned tuning, cudaStream_t st) {
 cudaError_t launch_half(const PsRun& P, unsigned tuning, cudaStream_t st) {
   cudaError_t e = init_constants();
   if (e != cudaSuccess) return e;
-  const bool tex = (tuning & 0x2u) != 0;
-  const int mode = half_mode(tuning, P.wr, P.ws);
-  if (mode != 0) {
-    const size_t smem = half_smem(P.wr, P.ws, true, P.maxsrc, 1, mode);
-#define PS_CASE(a, b) \
-    if (P.wr == a && P.ws == b) return launch_half_pairs<a, b>(P, mode, tex, smem, st);
+  if (half_staged(tuning, P.wr, P.ws)) {
+    const size_t smem = half_smem(P.wr, P.ws, true, P.maxsrc, true);
+#define PS_CASE(a, b)                                                                               \
+    if (P.wr == a && P.ws == b)                                                                     \
+      return P.tmaps ? launch(k_half_st<a, b, true>, P.ntiles, PS_HALF_NT, smem, st, P)             \
+                     : launch(k_half_st<a, b, false>, P.ntiles, PS_HALF_NT, smem, st, P);
     PS_SPECS(PS_CASE)
 #undef PS_CASE
   }
-  const bool cw = use_cache(P.wr, P.ws) && !(tuning & 0x1u);
-  const int G = half_lanes(tuning);
-  const size_t smem = half_smem(P.wr, P.ws, cw, P.maxsrc, G, 0);
-#define PS_CASE(a, b)                                                                \
-  if (P.wr == a && P.ws == b)                                                        \
-    return G == 2 ? launch_half_g<a, b, 2>(P, cw, tex, smem, st) : launch_half_g<a, b, 1>(P, cw, tex, smem, st);
+  const bool cw = use_cache(P.wr, P.ws);
+  const size_t smem = half_smem(P.wr, P.ws, cw, P.maxsrc, false);
+#define PS_CASE(a, b) \
+  if (P.wr == a && P.ws == b) return launch(k_half<a, b, true>, P.ntiles, PS_HALF_NT, smem, st, P);
   PS_SPECS(PS_CASE)
 #undef PS_CASE
-  return G == 2 ? launch_half_g<0, 1, 2>(P, cw, tex, smem, st) : launch_half_g<0, 1, 1>(P, cw, tex, smem, st);
+  // Any other window: four columns unrolled and four CTAs per SM while at least three weight caches fit there (up to 11
+  // columns) or without the cache, else eight columns and two CTAs (ms per half step, first against second form: 9×9
+  // 4.34 / 5.21, 15×15 step 2 3.29 / 3.69, 15×15 step 1 29.9 / 20.6, 17×17 35.9 / 18.9, 21×21 uncached 41.1 / 70.8).
+  if (!cw) return launch(k_half<0, 4, false>, P.ntiles, PS_HALF_NT, smem, st, P);
+  return 3 * (smem + 1024) <= 228 * 1024 ? launch(k_half<0, 4, true>, P.ntiles, PS_HALF_NT, smem, st, P)
+                                         : launch(k_half<0, 8, true>, P.ntiles, PS_HALF_NT, smem, st, P);
 }
 
-// tex: the session built texture objects for its planes (PS_TUNE_TEX_GATHER); the specialised windows then sample
-// through them, the generic kernels keep the plane loads.
-cudaError_t launch_eval(const PsRun& P, bool tex, cudaStream_t st) {
+cudaError_t launch_eval(const PsRun& P, cudaStream_t st) {
   const bool cw = use_cache(P.wr, P.ws);
   const size_t smem = eval_smem(P.wr, P.ws, cw);
-#define PS_CASE(a, b)                                                                                  \
-  if (P.wr == a && P.ws == b)                                                                          \
-    return tex ? launch(k_eval<a, b, true, true>, P.ntiles, PS_EVAL_NT, smem, st, P)                   \
-               : launch(k_eval<a, b, true, false>, P.ntiles, PS_EVAL_NT, smem, st, P);
+#define PS_CASE(a, b) \
+  if (P.wr == a && P.ws == b) return launch(k_eval<a, b, true>, P.ntiles, PS_EVAL_NT, smem, st, P);
   PS_SPECS(PS_CASE)
 #undef PS_CASE
-  if (cw) return launch(k_eval<0, 1, true, false>, P.ntiles, PS_EVAL_NT, smem, st, P);
-  return launch(k_eval<0, 1, false, false>, P.ntiles, PS_EVAL_NT, smem, st, P);
+  return cw ? launch(k_eval<0, 4, true>, P.ntiles, PS_EVAL_NT, smem, st, P)
+            : launch(k_eval<0, 4, false>, P.ntiles, PS_EVAL_NT, smem, st, P);
 }
 
-cudaError_t launch_filter(const PsRun& P, bool tex, cudaStream_t st) {
+cudaError_t launch_filter(const PsRun& P, cudaStream_t st) {
   const bool cw = use_cache(P.wr, P.ws);
   const size_t smem = eval_smem(P.wr, P.ws, cw);
-#define PS_CASE(a, b)                                                                                  \
-  if (P.wr == a && P.ws == b)                                                                          \
-    return tex ? launch(k_filter<a, b, true, true>, P.ntiles, PS_EVAL_NT, smem, st, P)                 \
-               : launch(k_filter<a, b, true, false>, P.ntiles, PS_EVAL_NT, smem, st, P);
+#define PS_CASE(a, b) \
+  if (P.wr == a && P.ws == b) return launch(k_filter<a, b, true>, P.ntiles, PS_EVAL_NT, smem, st, P);
   PS_SPECS(PS_CASE)
 #undef PS_CASE
-  if (cw) return launch(k_filter<0, 1, true, false>, P.ntiles, PS_EVAL_NT, smem, st, P);
-  return launch(k_filter<0, 1, false, false>, P.ntiles, PS_EVAL_NT, smem, st, P);
+  return cw ? launch(k_filter<0, 4, true>, P.ntiles, PS_EVAL_NT, smem, st, P)
+            : launch(k_filter<0, 4, false>, P.ntiles, PS_EVAL_NT, smem, st, P);
 }
-
 cudaError_t launch_upsample(const PsRun& P, cudaStream_t st) {
   if (P.ntiles <= 0) return cudaSuccess;
   k_upsample<<<P.ntiles, dim3(PS_SIMPLE_BX, PS_SIMPLE_BY), 0, st>>>(P);
@@ -2326,19 +2085,13 @@ cudaError_t launch_readout(const PsRun& P, float4* out, cudaStream_t st) {
 }
 size_t sweep_smem(int wr, int ws) { return eval_smem(wr, ws, true); }
 
-// `tex`: sample sources through their texture objects (tex2Dgather; same bits as the software bilinear).
-cudaError_t launch_sweep(const PsRun& P, bool tex, cudaStream_t st) {
+cudaError_t launch_sweep(const PsRun& P, cudaStream_t st) {
   const size_t smem = sweep_smem(P.wr, P.sweep_ws);
-  if (P.wr == 6 && P.sweep_ws == 2)
-    return tex ? launch(k_sweep<6, 2, true>, P.ntiles, PS_EVAL_NT, smem, st, P)
-               : launch(k_sweep<6, 2, false>, P.ntiles, PS_EVAL_NT, smem, st, P);
-  if (P.wr == 5 && P.sweep_ws == 2)
-    return tex ? launch(k_sweep<5, 2, true>, P.ntiles, PS_EVAL_NT, smem, st, P)
-               : launch(k_sweep<5, 2, false>, P.ntiles, PS_EVAL_NT, smem, st, P);
+  if (P.wr == 6 && P.sweep_ws == 2) return launch(k_sweep<6, 2>, P.ntiles, PS_EVAL_NT, smem, st, P);
+  if (P.wr == 5 && P.sweep_ws == 2) return launch(k_sweep<5, 2>, P.ntiles, PS_EVAL_NT, smem, st, P);
   PsRun Q = P;
   Q.ws = P.sweep_ws;  // the generic kernel reads the window step from the parameters
-  return tex ? launch(k_sweep<0, 1, true>, Q.ntiles, PS_EVAL_NT, smem, st, Q)
-             : launch(k_sweep<0, 1, false>, Q.ntiles, PS_EVAL_NT, smem, st, Q);
+  return launch(k_sweep<0, 4>, Q.ntiles, PS_EVAL_NT, smem, st, Q);
 }
 
 // Per-pixel restorer choice of the multi-scale driver (the host driver's `take` rule): the restorer run's plane stays

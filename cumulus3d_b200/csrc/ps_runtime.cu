@@ -34,14 +34,13 @@
   cudaError_t launch_half(const PsRun& P, unsigned tuning, cudaStream_t st);                               \
   bool half_run_ok(unsigned tuning, int wr, int ws);                                                       \
   cudaError_t launch_half_run(const PsRun& P, unsigned tuning, cudaStream_t st);                           \
-  int half_lanes(unsigned tuning);                                                                         \
-  cudaError_t launch_eval(const PsRun& P, bool tex, cudaStream_t st);                                      \
-  cudaError_t launch_filter(const PsRun& P, bool tex, cudaStream_t st);                                    \
+  cudaError_t launch_eval(const PsRun& P, cudaStream_t st);                                                \
+  cudaError_t launch_filter(const PsRun& P, cudaStream_t st);                                              \
   cudaError_t launch_upsample(const PsRun& P, cudaStream_t st);                                            \
   cudaError_t launch_median(const PsRun& P, cudaStream_t st);                                              \
   cudaError_t launch_snapshot(const PsRun& P, float* snap, cudaStream_t st);                               \
   cudaError_t launch_readout(const PsRun& P, float4* out, cudaStream_t st);                                \
-  cudaError_t launch_sweep(const PsRun& P, bool tex, cudaStream_t st);                                     \
+  cudaError_t launch_sweep(const PsRun& P, cudaStream_t st);                                               \
   cudaError_t launch_restore(const PsRun& P, const float4* up, const float* cinit, float thr, cudaStream_t st); \
   cudaError_t launch_fp32_probe(float* out, int blocks, int iters, cudaStream_t st);                       \
   cudaError_t launch_rcp_check(int e_lo, int e_hi, unsigned long long* bad, unsigned* first, cudaStream_t st); \
@@ -57,29 +56,28 @@ namespace {
 
 struct Launchers {
   cudaError_t (*half)(const PsRun&, unsigned, cudaStream_t);
-  cudaError_t (*eval)(const PsRun&, bool, cudaStream_t);
-  cudaError_t (*filter)(const PsRun&, bool, cudaStream_t);
+  cudaError_t (*eval)(const PsRun&, cudaStream_t);
+  cudaError_t (*filter)(const PsRun&, cudaStream_t);
   cudaError_t (*upsample)(const PsRun&, cudaStream_t);
   cudaError_t (*median)(const PsRun&, cudaStream_t);
   cudaError_t (*snapshot)(const PsRun&, float*, cudaStream_t);
   cudaError_t (*readout)(const PsRun&, float4*, cudaStream_t);
-  int (*half_lanes)(unsigned);
-  cudaError_t (*sweep)(const PsRun&, bool, cudaStream_t);
+  cudaError_t (*sweep)(const PsRun&, cudaStream_t);
   cudaError_t (*restore)(const PsRun&, const float4*, const float*, float, cudaStream_t);
   bool (*half_run_ok)(unsigned, int, int);
   cudaError_t (*half_run)(const PsRun&, unsigned, cudaStream_t);
 };
 const Launchers kParity = {ps_parity::launch_half,     ps_parity::launch_eval,   ps_parity::launch_filter,
                            ps_parity::launch_upsample, ps_parity::launch_median, ps_parity::launch_snapshot,
-                           ps_parity::launch_readout,  ps_parity::half_lanes,    ps_parity::launch_sweep,
+                           ps_parity::launch_readout,  ps_parity::launch_sweep,
                            ps_parity::launch_restore, ps_parity::half_run_ok, ps_parity::launch_half_run};
 const Launchers kFast = {ps_fast::launch_half,     ps_fast::launch_eval,   ps_fast::launch_filter,
                          ps_fast::launch_upsample, ps_fast::launch_median, ps_fast::launch_snapshot,
-                         ps_fast::launch_readout,  ps_fast::half_lanes,    ps_fast::launch_sweep,
+                         ps_fast::launch_readout,  ps_fast::launch_sweep,
                          ps_fast::launch_restore, ps_fast::half_run_ok, ps_fast::launch_half_run};
 const Launchers kChecked = {ps_checked::launch_half,     ps_checked::launch_eval,   ps_checked::launch_filter,
                             ps_checked::launch_upsample, ps_checked::launch_median, ps_checked::launch_snapshot,
-                            ps_checked::launch_readout,  ps_checked::half_lanes,    ps_checked::launch_sweep,
+                            ps_checked::launch_readout,  ps_checked::launch_sweep,
                             ps_checked::launch_restore, ps_checked::half_run_ok, ps_checked::launch_half_run};
 
 struct PsError {
@@ -229,7 +227,7 @@ struct ps_session {
   size_t pin_cap = 0;
   uint64_t launches = 0;
   size_t img_bytes = 0;
-  std::vector<cudaArray_t> arrays;       // texture arrays (PS_TUNE_TEX_GATHER)
+  std::vector<cudaArray_t> arrays;       // texture arrays
   std::vector<ps_backend::CachedArray> array_keys;  // their sizes and formats, handed back to the backend at the end
   std::vector<cudaTextureObject_t> texs;
   unsigned tuning = 0;
@@ -780,10 +778,9 @@ void run_batch(ps_session* s, const uint32_t* views, size_t a, size_t b, const p
     P.proposal = sl.proposal;
   }
   set_items(s, P, views, a, b, (int)p->level, PS_EVAL_PW, PS_EVAL_PH);
-  timed_launch(s, PS_KERNEL_EVAL, P, [&](const PsRun& q) { return s->L->eval(q, s->tuning & PS_TUNE_TEX_GATHER, s->st); }, "evaluate kernel");
+  timed_launch(s, PS_KERNEL_EVAL, P, [&](const PsRun& q) { return s->L->eval(q, s->st); }, "evaluate kernel");
   PsRun H = P;
-  set_items(s, H, views, a, b, (int)p->level, s->L->half_lanes(s->tuning) == 2 ? PS_HALF2_PW : PS_HALF_PW,
-            PS_HALF_PH);
+  set_items(s, H, views, a, b, (int)p->level, PS_HALF_PW, PS_HALF_PH);
   if (s->L->half_run_ok(s->tuning, H.wr, H.ws)) {
     // persistent kernel: up to PS_MAX_PHASES half steps per launch, over a zeroed queue
     for (uint32_t t0 = 0; t0 < p->iterations; t0 += PS_MAX_PHASES / 2) {
@@ -1059,7 +1056,7 @@ int ps_begin(ps_backend* be, const ps_kernel_input* in, ps_session** out) {
         L.cx = li.k[2];
         L.cy = li.k[3];
       }
-    if (s->tuning & PS_TUNE_TEX_GATHER) {
+    {
       // one gather-capable CUDA array + border-addressed point texture per (view, level).  8-bit images keep 8-bit
       // texels read as normalized floats (the texture unit returns the correctly rounded u/255, the plane's value, for
       // every u); f32 images are copied from the plane.
@@ -1458,7 +1455,7 @@ int ps_evaluate(ps_session* s, uint32_t level, const uint32_t* views, size_t n, 
       P.geometric = geometric ? 1 : 0;
       P.mode = 0;
       set_items(s, P, views, a, b, (int)level, PS_EVAL_PW, PS_EVAL_PH);
-      timed_launch(s, PS_KERNEL_EVAL, P, [&](const PsRun& q) { return s->L->eval(q, s->tuning & PS_TUNE_TEX_GATHER, s->st); }, "evaluate kernel");
+      timed_launch(s, PS_KERNEL_EVAL, P, [&](const PsRun& q) { return s->L->eval(q, s->st); }, "evaluate kernel");
       for (size_t i = a; i < b; ++i) {
         if (!out_cost[i]) fail(PS_EINVAL, "out_cost entry is NULL");
         cuda_ok(cudaMemcpyAsync(out_cost[i], sl.cost + sl.off[views[i]],
@@ -1484,7 +1481,7 @@ int ps_filter(ps_session* s, const uint32_t* views, size_t n, const ps_view_stat
       PsRun P = base_params(s, level);
       P.geometric = 1;
       set_items(s, P, views, a, b, level, PS_EVAL_PW, PS_EVAL_PH);
-      timed_launch(s, PS_KERNEL_FILTER, P, [&](const PsRun& q) { return s->L->filter(q, s->tuning & PS_TUNE_TEX_GATHER, s->st); }, "filter kernel");
+      timed_launch(s, PS_KERNEL_FILTER, P, [&](const PsRun& q) { return s->L->filter(q, s->st); }, "filter kernel");
       for (size_t i = a; i < b; ++i) {
         if (!out_counts[i]) fail(PS_EINVAL, "out_counts entry is NULL");
         cuda_ok(cudaMemcpyAsync(out_counts[i], sl.count + sl.off[views[i]],
@@ -1616,7 +1613,7 @@ int ps_filter_resident(ps_session* s, const uint32_t* views, size_t n, uint8_t* 
       PsRun P = base_params(s, level);
       P.geometric = 1;
       set_items(s, P, views, a, b, level, PS_EVAL_PW, PS_EVAL_PH);
-      timed_launch(s, PS_KERNEL_FILTER, P, [&](const PsRun& q) { return s->L->filter(q, s->tuning & PS_TUNE_TEX_GATHER, s->st); }, "filter kernel");
+      timed_launch(s, PS_KERNEL_FILTER, P, [&](const PsRun& q) { return s->L->filter(q, s->st); }, "filter kernel");
       if (out_counts) {
         for (size_t i = a; i < b; ++i)
           if (out_counts[i])
@@ -1676,7 +1673,7 @@ void enqueue_schedule(ps_session* s, const uint32_t* views, size_t n, const ps_s
     PsRun P = base_params(s, level);
     P.geometric = 1;
     set_items(s, P, views, a, b, level, PS_EVAL_PW, PS_EVAL_PH);
-    timed_launch(s, PS_KERNEL_FILTER, P, [&](const PsRun& q) { return s->L->filter(q, s->tuning & PS_TUNE_TEX_GATHER, s->st); }, "filter kernel");
+    timed_launch(s, PS_KERNEL_FILTER, P, [&](const PsRun& q) { return s->L->filter(q, s->st); }, "filter kernel");
     PsRun Q = base_params(s, level);
     set_items(s, Q, views, a, b, level, PS_SIMPLE_BX, PS_SIMPLE_BY);
     launched(s, s->L->readout(Q, sl.aux, s->st), "readout kernel");
@@ -1714,7 +1711,7 @@ void enqueue_multiscale(ps_session* s, const uint32_t* views, size_t n, const ps
         launched(s, s->L->upsample(U, s->st), "upsample kernel");
         PsRun E = base_params(s, l);  // c_init: top-K photometric cost of the upsampled planes
         set_items(s, E, views, a, b, l, PS_EVAL_PW, PS_EVAL_PH);
-        timed_launch(s, PS_KERNEL_EVAL, E, [&](const PsRun& q) { return s->L->eval(q, s->tuning & PS_TUNE_TEX_GATHER, s->st); }, "evaluate kernel");
+        timed_launch(s, PS_KERNEL_EVAL, E, [&](const PsRun& q) { return s->L->eval(q, s->st); }, "evaluate kernel");
       }
       for (size_t i = 0; i < n; ++i) {  // keep the upsampled planes and their cost
         const size_t np = (size_t)s->W(views[i], l) * s->H(views[i], l), o = (size_t)sl.off[views[i]];
@@ -1729,7 +1726,7 @@ void enqueue_multiscale(ps_session* s, const uint32_t* views, size_t n, const ps
       for (auto [a, b] : batches(s, views, n, l)) {
         PsRun E = base_params(s, l);  // c_photo
         set_items(s, E, views, a, b, l, PS_EVAL_PW, PS_EVAL_PH);
-        timed_launch(s, PS_KERNEL_EVAL, E, [&](const PsRun& q) { return s->L->eval(q, s->tuning & PS_TUNE_TEX_GATHER, s->st); }, "evaluate kernel");
+        timed_launch(s, PS_KERNEL_EVAL, E, [&](const PsRun& q) { return s->L->eval(q, s->st); }, "evaluate kernel");
         PsRun R = base_params(s, l);
         set_items(s, R, views, a, b, l, PS_SIMPLE_BX, PS_SIMPLE_BY);
         launched(s, s->L->restore(R, sl.aux, sl.cinit, m->restorer_threshold, s->st), "restore kernel");
@@ -1759,7 +1756,7 @@ void enqueue_multiscale(ps_session* s, const uint32_t* views, size_t n, const ps
     PsRun P = base_params(s, top);
     P.geometric = 1;
     set_items(s, P, views, a, b, top, PS_EVAL_PW, PS_EVAL_PH);
-    timed_launch(s, PS_KERNEL_FILTER, P, [&](const PsRun& q) { return s->L->filter(q, s->tuning & PS_TUNE_TEX_GATHER, s->st); }, "filter kernel");
+    timed_launch(s, PS_KERNEL_FILTER, P, [&](const PsRun& q) { return s->L->filter(q, s->st); }, "filter kernel");
     PsRun Q = base_params(s, top);
     set_items(s, Q, views, a, b, top, PS_SIMPLE_BX, PS_SIMPLE_BY);
     launched(s, s->L->readout(Q, st.aux, s->st), "readout kernel");
@@ -1953,8 +1950,7 @@ void enqueue_sweep(ps_session* s, int level, uint32_t view, unsigned short* out,
   P.sweep_ws = 2;
   for (int c = 0; c < 3; ++c) P.sweep_n[c] = s->sweep_n[3 * view + c];
   set_items(s, P, &view, 0, 1, level, PS_EVAL_PW, PS_EVAL_PH);
-  const bool tex = (s->tuning & PS_TUNE_TEX_GATHER) != 0;  // the session built texture objects for its planes
-  timed_launch(s, PS_KERNEL_SWEEP, P, [&](const PsRun& q) { return s->L->sweep(q, tex, s->st); }, "sweep kernel");
+  timed_launch(s, PS_KERNEL_SWEEP, P, [&](const PsRun& q) { return s->L->sweep(q, s->st); }, "sweep kernel");
 }
 
 template <typename T>

@@ -12,7 +12,6 @@
 // Half-step CTA: 128 threads, 4 warps; a warp covers 16 active columns × 2 rows of a 32 × 8 pixel tile.
 #define PS_HALF_NT 128
 #define PS_HALF_PW 32
-#define PS_HALF2_PW 16  // two lanes per pixel: a warp = 8 active columns × 2 rows × 2 lanes
 #define PS_HALF_PH 8
 // Staged-source half step (PS_TUNE_STAGED): a warp covers an 8 × 8 pixel block (4 active columns × 8 rows) of the
 // 32 × 8 tile and stages the union of its lanes' source footprints of one window into a PS_BOX_P × PS_BOX_H box of
@@ -57,7 +56,7 @@ enum PsCheckSite {
 // One (view, level) image plane.
 struct PsLevel {
   const float* img;    // pixel (0,0) of a plane with PS_BORDER zero rows/columns on every side
-  unsigned long long tex;  // border-addressed point texture of the same plane (cudaTextureObject_t), 0 if not built
+  unsigned long long tex;  // border-addressed point texture of the same plane (cudaTextureObject_t)
   int w, h, pitch;         // pitch in floats
   int pad;
   float fx, fy, cx, cy;

@@ -72,12 +72,14 @@ typedef struct ps_options {
   uint32_t tuning;       /* half-step kernel variant, PS_TUNE_* flags; 0 = defaults (the autotuner sets these) */
 } ps_options;
 
-/* Half-step kernel variants (same results bit for bit; only speed differs). */
-#define PS_TUNE_NO_WEIGHT_CACHE 0x1u /* recompute window weights per tap (more CTAs per SM, more exp work) */
-#define PS_TUNE_TEX_GATHER 0x2u      /* fetch each bilinear 2×2 footprint with one texture gather (same bits) */
-#define PS_TUNE_ONE_LANE 0x4u        /* one thread per pixel (default: two lanes per pixel split the window rows) */
-#define PS_TUNE_ROW_PAIRS 0x8u       /* one thread per pixel, window rows 2p and 2p+1 as packed f32x2 pairs */
-#define PS_TUNE_STAGED 0x10u         /* row pairs, and each warp stages its sources' footprints in shared memory */
+/* Half-step kernel variants (same results bit for bit; only speed differs).  The default is one thread per pixel, window
+ * rows 2p and 2p+1 as packed f32x2 pairs, each bilinear 2×2 footprint fetched with one texture gather.  The first four
+ * flags are accepted and select that same kernel: it is the fastest at every window and size. */
+#define PS_TUNE_NO_WEIGHT_CACHE 0x1u
+#define PS_TUNE_TEX_GATHER 0x2u
+#define PS_TUNE_ONE_LANE 0x4u
+#define PS_TUNE_ROW_PAIRS 0x8u
+#define PS_TUNE_STAGED 0x10u         /* each warp stages its sources' footprints in shared memory (compiled windows) */
 #define PS_TUNE_PERSISTENT 0x20u     /* with PS_TUNE_ROW_PAIRS: one persistent launch per run over a device work queue of
                                         (half step, tile) items with bounded per-view waits between half steps; a
                                         wait that gives up fails the call with PS_ETIMEOUT */
