@@ -4,7 +4,7 @@
 //   * 3×3 convolution forward as an implicit GEMM on the tensor cores (mma.sync m16n8k16, BF16 operands, FP32
 //     accumulation), bias and ReLU fused into the epilogue; the data gradient is the same kernel run with the
 //     weights flipped in space and transposed in channels;
-//   * 3×3 convolution weight gradient as a split-K implicit GEMM (tensor cores, FP32 atomics across pixel chunks);
+//   * 3×3 convolution weight gradient as a split-K implicit GEMM over halo tiles (tensor cores, FP32 reductions per CTA);
 //   * 2×2 average pooling, nearest 2× upsampling, channel concat and their gradients, the loss and its gradient,
 //     AdamW on FP32 master weights with BF16 copies for the forward pass.
 // Layout: activations NHWC in BF16 with channel counts that are multiples of 16; weights [Cout][9][Cin] (K-major).
@@ -34,9 +34,7 @@ namespace ps_cnn {
 
 // ------------------------------------------------------------------------------------------- tensor-core tiles
 // Convolution as an implicit GEMM: C[p][co] = sum_{tap, ci} X[p shifted by tap][ci] * W[co][tap][ci] (M = pixels,
-// N = cout, K = 9·cin) on mma.sync m16n8k16 (bf16 operands, f32 accumulators).  Weight-gradient tile (k_conv_wgrad):
-// 128 threads, 64 × 64 outputs, K in chunks of 16 pixels; warps 2 × 2, each 32 × 32 = 2 (m16) × 4 (n8) fragments.
-constexpr int CM = 64, CN = 64, CK = 16, CPAD = 8;
+// N = cout, K = 9·cin) on mma.sync m16n8k16 (bf16 operands, f32 accumulators).
 
 __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, const uint32_t* b) {
   asm volatile(
@@ -54,7 +52,10 @@ struct ConvArgs {
   float* yf;       // [B][H][W][cout] (f32 output) or null
   int B, H, W, cin, cin_stride, cin_off, cout;
   int relu;
-  // Virtual "upsample + concatenate" input (k_conv2 only; x2 == null: off): input channels [0, split) are x at half
+  // Output positions where mask [B][H][W][cout] is not positive become 0 (the ReLU of the layer below, in the data
+  // gradient); null: off.  bf16 output only.
+  const bf16* mask;
+  // Virtual "upsample + concatenate" input (x2 == null: off): input channels [0, split) are x at half
   // resolution [B][H/2][W/2][cin_stride] read at (y/2, x/2) (nearest 2× upsampling), channels [split, cin) are
   // x2 [B][H][W][x2_stride] (the skip connection).  split is a multiple of 8.
   const bf16* x2;
@@ -198,6 +199,11 @@ __global__ void __launch_bounds__(256) k_conv2(ConvArgs a) {
       if (a.relu) {
         v0 = fmaxf(v0, 0.f);
         v1 = fmaxf(v1, 0.f);
+      }
+      if (a.mask) {
+        const __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(a.mask + p * a.cout + co);
+        if (!(__low2float(m) > 0.f)) v0 = 0.f;
+        if (!(__high2float(m) > 0.f)) v1 = 0.f;
       }
       if (a.y) *reinterpret_cast<__nv_bfloat162*>(a.y + p * a.cout + co) = __floats2bfloat162_rn(v0, v1);
       if (a.yf) *reinterpret_cast<float2*>(a.yf + p * a.cout + co) = make_float2(v0, v1);
@@ -421,6 +427,13 @@ __global__ void __launch_bounds__(128, 1) k_conv5(ConvArgs a) {
               v[e] = __uint_as_float(v32[j + e]) + (a.bias ? a.bias[c0 + j + e] : 0.f);
               if (a.relu) v[e] = fmaxf(v[e], 0.f);
             }
+            if (a.mask) {
+              const uint4 mq = *reinterpret_cast<const uint4*>(a.mask + p * a.cout + c0 + j);
+              const bf16* m = reinterpret_cast<const bf16*>(&mq);
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+                if (!(__bfloat162float(m[e]) > 0.f)) v[e] = 0.f;
+            }
             if (a.y) {
               uint4 o;
               __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(&o);
@@ -445,95 +458,135 @@ __global__ void __launch_bounds__(128, 1) k_conv5(ConvArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------- conv weight gradient
-// dW[co][tap][ci] += sum_p dY[p][co] * X[p shifted by tap][ci];  M = Cout, N = 9·Cin (n = tap·Cin + ci), K = pixels.
-// Each CTA reduces a chunk of `pix_per_cta` pixels and adds its 64×64 tile into dW with FP32 atomics.
+// dW[co][tap][ci] += sum_p dY[p][co] * X[p shifted by tap][ci]: M = cout, N = (tap, ci), K = pixels.  A CTA of 9 warps
+// owns 16·MT output channels × 32 input channels × the 9 taps and walks every gridDim.z-th 8 × 16 pixel tile: it stages
+// the tile's dY rows and the (8+2) × (16+2) halo of X with cp.async into a double buffer, and warp `tap` multiplies the
+// tile's rows (16 pixels = one K step) against the halo shifted by its tap.  Both operands lie pixel-major in shared
+// memory, so the fragments come through ldmatrix.trans (rows padded to an odd multiple of 16 bytes: no bank conflicts),
+// and the 9 taps share one copy of X.  The sums stay in FP32 registers over all tiles of the CTA, and are added to dW
+// with one vector reduction per pair at the end.
+//
+// What bounds it is the tensor pipe of mma.sync.  The earlier form (64 × 64 outputs, K chunks of 16 pixels gathered
+// element by element, a division per element) and the one-element kernels around it took a training step of batch 8 at
+// 256 × 256 to 28.5 ms; with this one, masks fused into the convolutions and 16-byte accesses it takes 3.3 ms.
 struct WgradArgs {
   const bf16* dy;  // [P][cout]
-  const bf16* x;   // [B][H][W][cin_stride] (+cin_off)
-  float* dw;       // [cout][9][cin]
-  int B, H, W, cin, cin_stride, cin_off, cout, pix_per_cta;
+  const bf16* x;   // [B][H][W][cin_stride], or (x2 != null) the half-resolution part of a virtual concatenation
+  const bf16* x2;  // as in ConvArgs
+  float* dw;       // [cout][9][cin], 8-byte aligned
+  int B, H, W, cin, cin_stride, cout, split, x2_stride;
+};
+constexpr int WG_CI = 32, WG_XP = WG_CI + 8, WG_NT = 9 * 32;
+template <int MT>
+struct WgCfg {
+  static constexpr int CO = 16 * MT, DP = CO + 8;
+  static constexpr int stage = HALO_PX * WG_XP + HT_H * HT_W * DP;  // bf16 elements
+  static constexpr size_t smem = (size_t)2 * stage * sizeof(bf16);
 };
 
-__global__ void __launch_bounds__(128) k_conv_wgrad(WgradArgs a) {
-  __shared__ __align__(16) bf16 As[CM][CK + CPAD];  // [co][p]
-  __shared__ __align__(16) bf16 Bs[CN][CK + CPAD];  // [n][p]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp >> 1, wn = warp & 1;
-  const int co0 = blockIdx.x * CM;
-  const int nk = 9 * a.cin;
-  const int n0 = blockIdx.y * CN;
-  const long long P = (long long)a.B * a.H * a.W;
-  const long long pbeg = (long long)blockIdx.z * a.pix_per_cta;
-  const long long pend = min(P, pbeg + a.pix_per_cta);
-  float acc[2][4][4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) acc[i][j][k] = 0.f;
-  for (long long pc = pbeg; pc < pend; pc += CK) {
-    // A: As[co][pp] = dY[pc+pp][co0+co]; 64 × 16 -> each thread 8 values
-    for (int e = tid; e < CM * CK; e += 128) {
-      const int pp = e / CM, co = e % CM;
-      const long long p = pc + pp;
-      bf16 v = __float2bfloat16(0.f);
-      if (p < pend && co0 + co < a.cout) v = a.dy[p * a.cout + co0 + co];
-      As[co][pp] = v;
-    }
-    // B: Bs[n][pp] = X[pc+pp shifted by tap(n)][ci(n)]
-    for (int e = tid; e < CN * CK; e += 128) {
-      const int pp = e / CN, nn = e % CN;
-      const long long p = pc + pp;
-      const int n = n0 + nn;
-      bf16 v = __float2bfloat16(0.f);
-      if (p < pend && n < nk) {
-        const int tap = n / a.cin, ci = n - tap * a.cin;
-        const int b = (int)(p / ((long long)a.H * a.W));
-        const int rem = (int)(p - (long long)b * a.H * a.W);
-        const int y = rem / a.W + tap / 3 - 1, x = rem % a.W + tap % 3 - 1;
-        if (y >= 0 && y < a.H && x >= 0 && x < a.W)
-          v = a.x[(((long long)b * a.H + y) * a.W + x) * a.cin_stride + a.cin_off + ci];
+__device__ __forceinline__ void ldsm_x4_t(uint32_t* r, const void* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(smem_u32(p)));
+}
+
+template <int MT>
+__global__ void __launch_bounds__(WG_NT, 2) k_conv_wgrad(WgradArgs a) {
+  using Cfg = WgCfg<MT>;
+  constexpr int CO = Cfg::CO, DP = Cfg::DP;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  bf16* sm = reinterpret_cast<bf16*>(smraw);
+  const int tid = threadIdx.x, tap = tid >> 5, lane = tid & 31;
+  const int dy = tap / 3, dx = tap - dy * 3;
+  const int co0 = blockIdx.x * CO, ci0 = blockIdx.y * WG_CI;
+  const int tiles_x = (a.W + HT_W - 1) / HT_W, tiles_y = (a.H + HT_H - 1) / HT_H;
+  const int ntiles = a.B * tiles_x * tiles_y;
+
+  auto load_stage = [&](int stage, int t) {
+    const int b = t / (tiles_x * tiles_y);
+    t -= b * tiles_x * tiles_y;
+    const int ty0 = (t / tiles_x) * HT_H, tx0 = (t % tiles_x) * HT_W;
+    bf16* halo = sm + (size_t)stage * Cfg::stage;
+    bf16* ds = halo + HALO_PX * WG_XP;
+    for (int i = tid; i < HALO_PX * (WG_CI / 8); i += WG_NT) {
+      const int px = i / (WG_CI / 8), seg = i % (WG_CI / 8);
+      const int hy = px / HALO_W, hx = px - hy * HALO_W;
+      const int gy = ty0 + hy - 1, gx = tx0 + hx - 1, ch = ci0 + seg * 8;
+      const bool ok = gy >= 0 && gy < a.H && gx >= 0 && gx < a.W && ch < a.cin;
+      const bf16* src = a.x;
+      if (ok) {
+        if (!a.x2)
+          src = a.x + (((long long)b * a.H + gy) * a.W + gx) * a.cin_stride + ch;
+        else if (ch < a.split)
+          src = a.x + (((long long)b * (a.H >> 1) + (gy >> 1)) * (a.W >> 1) + (gx >> 1)) * a.cin_stride + ch;
+        else
+          src = a.x2 + (((long long)b * a.H + gy) * a.W + gx) * a.x2_stride + (ch - a.split);
       }
-      Bs[nn][pp] = v;
+      cp_async16(halo + px * WG_XP + seg * 8, src, ok ? 16 : 0);
+    }
+    for (int i = tid; i < HT_H * HT_W * (CO / 8); i += WG_NT) {
+      const int px = i / (CO / 8), seg = i % (CO / 8);
+      const int gy = ty0 + px / HT_W, gx = tx0 + px % HT_W, ch = co0 + seg * 8;
+      const bool ok = gy < a.H && gx < a.W && ch < a.cout;
+      cp_async16(ds + px * DP + seg * 8, ok ? a.dy + (((long long)b * a.H + gy) * a.W + gx) * a.cout + ch : a.dy,
+                 ok ? 16 : 0);
+    }
+    cp_async_commit();
+  };
+
+  float acc[MT][WG_CI / 8][4];
+#pragma unroll
+  for (int i = 0; i < MT; ++i)
+#pragma unroll
+    for (int j = 0; j < WG_CI / 8; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+
+  const int mat = lane >> 3, r8 = lane & 7;
+  int st = 0;
+  if ((int)blockIdx.z < ntiles) load_stage(0, blockIdx.z);
+  for (int t = blockIdx.z; t < ntiles; t += gridDim.z, st ^= 1) {
+    if (t + (int)gridDim.z < ntiles) {
+      load_stage(st ^ 1, t + gridDim.z);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
     }
     __syncthreads();
-    const int g = lane >> 2, t = lane & 3;
-    uint32_t af[2][4], bfr[4][2];
+    const bf16* halo = sm + (size_t)st * Cfg::stage;
+    const bf16* ds = halo + HALO_PX * WG_XP;
+#pragma unroll 2
+    for (int ry = 0; ry < HT_H; ++ry) {
+      uint32_t bq[WG_CI / 16][4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int r = wm * 32 + i * 16 + g;
-      af[i][0] = *(const uint32_t*)&As[r][t * 2];
-      af[i][1] = *(const uint32_t*)&As[r + 8][t * 2];
-      af[i][2] = *(const uint32_t*)&As[r][t * 2 + 8];
-      af[i][3] = *(const uint32_t*)&As[r + 8][t * 2 + 8];
+      for (int j = 0; j < WG_CI / 16; ++j)
+        ldsm_x4_t(bq[j], halo + ((ry + dy) * HALO_W + dx + (mat & 1) * 8 + r8) * WG_XP + j * 16 + (mat >> 1) * 8);
+#pragma unroll
+      for (int i = 0; i < MT; ++i) {
+        uint32_t af[4];
+        ldsm_x4_t(af, ds + (ry * HT_W + (mat >> 1) * 8 + r8) * DP + i * 16 + (mat & 1) * 8);
+#pragma unroll
+        for (int j = 0; j < WG_CI / 8; ++j) mma_bf16(acc[i][j], af, bq[j >> 1] + 2 * (j & 1));
+      }
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = wn * 32 + j * 8 + g;
-      bfr[j][0] = *(const uint32_t*)&Bs[c][t * 2];
-      bfr[j][1] = *(const uint32_t*)&Bs[c][t * 2 + 8];
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) mma_bf16(acc[i][j], af[i], bfr[j]);
-    __syncthreads();
+    __syncthreads();  // every warp is done with this stage before the prefetch after next overwrites it
   }
-  const int g = lane >> 2, t = lane & 3;
+  const int g = lane >> 2, tq = lane & 3;
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int i = 0; i < MT; ++i)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int co = co0 + wm * 32 + i * 16 + g + h * 8;
+      const int co = co0 + i * 16 + g + h * 8;
       if (co >= a.cout) continue;
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int n = n0 + wn * 32 + j * 8 + t * 2 + e;
-          if (n < nk) atomicAdd(a.dw + (long long)co * nk + n, acc[i][j][h * 2 + e]);
-        }
+      for (int j = 0; j < WG_CI / 8; ++j) {
+        const int ci = ci0 + j * 8 + tq * 2;  // cin is even: ci + 1 < cin whenever ci < cin
+        if (ci < a.cin)
+          asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(
+                           a.dw + ((long long)co * 9 + tap) * a.cin + ci),
+                       "f"(acc[i][j][h * 2]), "f"(acc[i][j][h * 2 + 1])
+                       : "memory");
+      }
     }
 }
 
@@ -547,23 +600,27 @@ __global__ void k_flip_weights(const bf16* w, bf16* wt, int cout, int cin) {
   wt[((long long)ci * 9 + (8 - tap)) * cout + co] = w[i];
 }
 
-// dY ⊙ (Y > 0) for a ReLU layer (in place on dY).
-__global__ void k_relu_bwd(bf16* dy, const bf16* y, long long n) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (!(__bfloat162float(y[i]) > 0.f)) dy[i] = __float2bfloat16(0.f);
-}
-
-// db[c] += sum_p dY[p][c]
-__global__ void k_bias_grad(const bf16* dy, float* db, long long P, int C) {
-  const int c = threadIdx.x % C;
-  const int lanes = blockDim.x / C;
-  const int sub = threadIdx.x / C;
-  if (sub >= lanes) return;
-  float s = 0.f;
-  for (long long p = (long long)blockIdx.x * lanes + sub; p < P; p += (long long)gridDim.x * lanes)
-    s += __bfloat162float(dy[p * C + c]);
-  atomicAdd(db + c, s);
+// db[c] += sum_p dY[p][c], eight channels per thread; C is a multiple of 8, at most 2048.
+__global__ void __launch_bounds__(256) k_bias_grad(const bf16* dy, float* db, long long P, int C) {
+  __shared__ float part[256][9];
+  const int C8 = C / 8, lanes = 256 / C8;
+  const int c8 = threadIdx.x % C8, sub = threadIdx.x / C8;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (sub < lanes)
+    for (long long p = (long long)blockIdx.x * lanes + sub; p < P; p += (long long)gridDim.x * lanes) {
+      const uint4 q = *reinterpret_cast<const uint4*>(dy + p * C + c8 * 8);
+      const bf16* e = reinterpret_cast<const bf16*>(&q);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) s[k] += __bfloat162float(e[k]);
+    }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) part[threadIdx.x][k] = s[k];
+  __syncthreads();
+  for (int c = threadIdx.x; c < C; c += 256) {
+    float t = 0.f;
+    for (int l = 0; l < lanes; ++l) t += part[l * C8 + c / 8][c & 7];
+    atomicAdd(db + c, t);
+  }
 }
 
 // 2×2 average pooling (NHWC) and its gradient.
@@ -587,64 +644,72 @@ __global__ void k_pool_fwd(const bf16* x, bf16* y, int B, int H, int W, int C) {
                                      __bfloat162float(e[3][k])));
   *(uint4*)(y + p * C + c) = o;
 }
-// dX (full res, C channels) = dY/4 broadcast; `accumulate` adds to dX.
-__global__ void k_pool_bwd(const bf16* dy, bf16* dx, int B, int H, int W, int C, int accumulate) {
+// Gradients below a skip connection, eight channels per thread (16-byte accesses; C, Cy and off are multiples of 8).
+//
+// At the encoder side: dS = (skip part of dC + dP/4 broadcast) where S > 0, else 0.  dC [B][H][W][Cy] holds the skip at
+// channels [off, off + C), dP [B][H/2][W/2][C] is the gradient of the 2×2 average pool, S the layer's output.
+__global__ void __launch_bounds__(256) k_skip_bwd(const bf16* dc, int Cy, int off, const bf16* dp, const bf16* s, bf16* ds,
+                                                  int B, int H, int W, int C) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)B * H * W * C) return;
-  const int c = i % C;
-  const long long p = i / C;
-  const int x = p % W, y = (p / W) % H, b = (int)(p / ((long long)W * H));
-  float v = 0.25f * __bfloat162float(dy[(((long long)b * (H / 2) + y / 2) * (W / 2) + x / 2) * C + c]);
-  if (accumulate) v += __bfloat162float(dx[i]);
-  dx[i] = __float2bfloat16(v);
+  const int C8 = C / 8;
+  if (i >= (long long)B * H * W * C8) return;
+  const int c = (int)(i % C8) * 8;
+  const long long p = i / C8;
+  const int x = (int)(p % W), y = (int)((p / W) % H), b = (int)(p / ((long long)W * H));
+  const uint4 q[3] = {*(const uint4*)(dc + p * Cy + off + c),
+                      *(const uint4*)(dp + (((long long)b * (H / 2) + y / 2) * (W / 2) + x / 2) * C + c),
+                      *(const uint4*)(s + p * C + c)};
+  const bf16 *e0 = (const bf16*)&q[0], *e1 = (const bf16*)&q[1], *e2 = (const bf16*)&q[2];
+  uint4 o;
+  bf16* r = (bf16*)&o;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const bf16 v = __float2bfloat16(0.25f * __bfloat162float(e1[k]) + __bfloat162float(e0[k]));
+    r[k] = __bfloat162float(e2[k]) > 0.f ? v : __float2bfloat16(0.f);
+  }
+  *(uint4*)(ds + p * C + c) = o;
 }
-// nearest 2× upsampling of x [B][H/2][W/2][C] into channels [0, C) of y [B][H][W][Cy]; gradient sums the 2×2 block.
-__global__ void k_up_fwd(const bf16* x, bf16* y, int B, int H, int W, int C, int Cy) {
+// At the decoder side (nearest 2× upsampling into channels [0, C) of the concatenation): dX = the 2×2 block sum of dC
+// where X > 0, else 0.
+__global__ void __launch_bounds__(256) k_up_bwd(const bf16* dc, const bf16* x, bf16* dx, int B, int H, int W, int C,
+                                                int Cy) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)B * H * W * C) return;
-  const int c = i % C;
-  const long long p = i / C;
-  const int xx = p % W, yy = (p / W) % H, b = (int)(p / ((long long)W * H));
-  y[p * Cy + c] = x[(((long long)b * (H / 2) + yy / 2) * (W / 2) + xx / 2) * C + c];
-}
-__global__ void k_up_bwd(const bf16* dy, bf16* dx, int B, int H, int W, int C, int Cy) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int h = H / 2, w = W / 2;
-  if (i >= (long long)B * h * w * C) return;
-  const int c = i % C;
-  const long long p = i / C;
-  const int xx = p % w, yy = (p / w) % h, b = (int)(p / ((long long)w * h));
-  float s = 0.f;
-  for (int dy2 = 0; dy2 < 2; ++dy2)
-    for (int dx2 = 0; dx2 < 2; ++dx2)
-      s += __bfloat162float(dy[(((long long)b * H + 2 * yy + dy2) * W + 2 * xx + dx2) * Cy + c]);
-  dx[i] = __float2bfloat16(s);
-}
-// channel copy: dst[p][doff + c] = src[p][soff + c] (optionally accumulating into dst)
-__global__ void k_copy_ch(const bf16* src, int sC, int soff, bf16* dst, int dC, int doff, int C, long long P, int accumulate) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= P * C) return;
-  const int c = i % C;
-  const long long p = i / C;
-  float v = __bfloat162float(src[p * sC + soff + c]);
-  if (accumulate) v += __bfloat162float(dst[p * dC + doff + c]);
-  dst[p * dC + doff + c] = __float2bfloat16(v);
+  const int h = H / 2, w = W / 2, C8 = C / 8;
+  if (i >= (long long)B * h * w * C8) return;
+  const int c = (int)(i % C8) * 8;
+  const long long p = i / C8;
+  const int xx = (int)(p % w), yy = (int)((p / w) % h), b = (int)(p / ((long long)w * h));
+  const bf16* src = dc + (((long long)b * H + 2 * yy) * W + 2 * xx) * Cy + c;
+  const uint4 q[5] = {*(const uint4*)src, *(const uint4*)(src + Cy), *(const uint4*)(src + (long long)W * Cy),
+                      *(const uint4*)(src + (long long)W * Cy + Cy), *(const uint4*)(x + p * C + c)};
+  uint4 o;
+  bf16* r = (bf16*)&o;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sum += __bfloat162float(((const bf16*)&q[j])[k]);
+    r[k] = __float2bfloat16(__bfloat162float(((const bf16*)&q[4])[k]) > 0.f ? sum : 0.f);
+  }
+  *(uint4*)(dx + p * C + c) = o;
 }
 
 __device__ __forceinline__ float sigm(float x) { return 1.f / (1.f + expf(-x)); }
 
 // Loss and gradient of the head output o [P][8] (f32) against labels [P][6]: (target normalised inverse depth
 // t* = (1/d* - 1/dmax) / (1/dmin - 1/dmax), normal xyz, valid, target depth d*).  Loss per valid pixel: |t - t*| + (1 - n̂·n*) + 0.5·BCE(conf, |d - d*| < 1 % d*).
-// Writes dO (bf16) scaled by 1/valid_count and adds the loss sum and the valid count to stats[0..1].
-__global__ void k_loss(const float* o, const float* lab, bf16* dout, float* stats, long long P, float inv_n,
-                       float inv_near, float inv_far) {
+// Writes dO (bf16, the gradient's bf16 value divided by the valid count stats[2]) and adds the loss sum and the valid
+// count to stats[0..1], once per block (an addition per pixel to the same two words took as long as a layer).
+__global__ void __launch_bounds__(256) k_loss(const float* o, const float* lab, bf16* dout, float* stats, long long P,
+                                              float inv_near, float inv_far) {
+  __shared__ float part[2][8];
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= P) return;
-  const float* L = lab + p * 6;
-  const float* O = o + p * 8;
+  const bool in = p < P;
+  const float* L = lab + (in ? p : 0) * 6;
+  const float* O = o + (in ? p : 0) * 8;
   float g[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   float loss = 0.f, valid = 0.f;
-  if (L[4] > 0.5f) {
+  if (in && L[4] > 0.5f) {
     valid = 1.f;
     const float t = sigm(O[0]);
     const float dt = t - L[0];
@@ -665,10 +730,29 @@ __global__ void k_loss(const float* o, const float* lab, bf16* dout, float* stat
     loss += -0.5f * (target * logf(fmaxf(cf, 1e-7f)) + (1.f - target) * logf(fmaxf(1.f - cf, 1e-7f)));
     g[4] = 0.5f * (cf - target);
   }
-  for (int k = 0; k < 8; ++k) dout[p * 8 + k] = __float2bfloat16(g[k] * inv_n);
-  if (valid > 0.f) {
-    atomicAdd(stats, loss);
-    atomicAdd(stats + 1, 1.f);
+  if (in) {
+    const float c = stats[2];
+    uint4 q;
+    bf16* r = (bf16*)&q;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      r[k] = __float2bfloat16(c > 0.f ? __bfloat162float(__float2bfloat16(g[k])) / c : 0.f);
+    *(uint4*)(dout + p * 8) = q;
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    loss += __shfl_down_sync(0xffffffffu, loss, d);
+    valid += __shfl_down_sync(0xffffffffu, valid, d);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    part[0][threadIdx.x >> 5] = loss;
+    part[1][threadIdx.x >> 5] = valid;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    float t = 0.f;
+    for (int k = 0; k < 8; ++k) t += part[threadIdx.x][k];
+    if (t != 0.f) atomicAdd(stats + threadIdx.x, t);
   }
 }
 
@@ -732,14 +816,6 @@ __global__ void k_count_valid(const float* lab, long long P, float* count) {
   if ((threadIdx.x & 31) == 0 && m) atomicAdd(count, (float)__popc(m));
 }
 
-// Scales the loss gradient by 1 / count (count read on the device: no host round trip inside a training step).
-__global__ void k_scale_grad(bf16* g, long long n, const float* count) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float c = *count;
-  g[i] = __float2bfloat16(c > 0.f ? __bfloat162float(g[i]) / c : 0.f);
-}
-
 // ------------------------------------------------------------------------------------------- host side
 struct Layer {
   int cin, cout;
@@ -781,13 +857,6 @@ const int kLayers[12][2] = {{48, 32}, {32, 32}, {32, 64}, {64, 64}, {64, 96}, {9
 enum { E0A, E0B, E1A, E1B, E2A, E2B, E3A, E3B, D2, D1, D0, HEAD };
 
 inline unsigned blocks(long long n, int t = 256) { return (unsigned)((n + t - 1) / t); }
-// Pixels per CTA of the weight gradient: at least `min_chunk`, a multiple of 16, and few enough chunks for grid.z.
-inline int wgrad_chunk(long long P, int min_chunk) {
-  long long c = (P + 65534) / 65535;
-  c = (c + 15) / 16 * 16;
-  return (int)(c > min_chunk ? c : min_chunk);
-}
-
 struct Fail {
   int code;
   std::string msg;
@@ -802,7 +871,7 @@ void ck(cudaError_t e, const char* what) {
 
 // Activation buffers of one pass at batch B and size H × W (multiples of 8), and their gradients for training.
 struct Acts {
-  bf16 *x, *a0, *s0, *p1, *a1, *s1, *p2, *a2, *s2, *p3, *a3, *b3, *c2, *d2, *c1, *d1, *c0, *d0;
+  bf16 *x, *a0, *s0, *p1, *a1, *s1, *p2, *a2, *s2, *p3, *a3, *b3, *d2, *d1, *d0;
   float* o;
   bf16 *g_o, *g_d0, *g_c0, *g_s0, *g_d1, *g_c1, *g_s1, *g_d2, *g_c2, *g_s2, *g_b3, *g_a3, *g_p3, *g_a2, *g_p2, *g_a1,
       *g_p1, *g_a0;
@@ -837,11 +906,8 @@ void carve(Net& n, int B, int H, int W, Acts* A, bool grads, bool own_io, cudaSt
   add(&a.p3, P3 * 96, 2);
   add(&a.a3, P3 * 128, 2);
   add(&a.b3, P3 * 128, 2);
-  if (grads) add(&a.c2, P2 * 224, 2);
   add(&a.d2, P2 * 96, 2);
-  if (grads) add(&a.c1, P1 * 160, 2);
   add(&a.d1, P1 * 64, 2);
-  if (grads) add(&a.c0, P0 * 96, 2);
   add(&a.d0, P0 * 32, 2);
   if (grads) {
     add(&a.g_o, P0 * 8, 2);
@@ -990,46 +1056,55 @@ void forward(Net& n, const Acts& a, int B, int H, int W, cudaStream_t st) {
   k_pool_fwd<<<blocks(P3 * 12), 256, 0, st>>>(a.s2, a.p3, B, H2, W2, 96);
   conv(n, st, E3A, a.p3, 96, a.a3, nullptr, B, H3, W3, 1);
   conv(n, st, E3B, a.a3, 128, a.b3, nullptr, B, H3, W3, 1);
-  if (a.c2) {  // training: the concatenations are materialised (the backward pass reads them)
-    k_up_fwd<<<blocks(P2 * 128), 256, 0, st>>>(a.b3, a.c2, B, H2, W2, 128, 224);
-    k_copy_ch<<<blocks(P2 * 96), 256, 0, st>>>(a.s2, 96, 0, a.c2, 224, 128, 96, P2, 0);
-    conv(n, st, D2, a.c2, 224, a.d2, nullptr, B, H2, W2, 1);
-    k_up_fwd<<<blocks(P1 * 96), 256, 0, st>>>(a.d2, a.c1, B, H1, W1, 96, 160);
-    k_copy_ch<<<blocks(P1 * 64), 256, 0, st>>>(a.s1, 64, 0, a.c1, 160, 96, 64, P1, 0);
-    conv(n, st, D1, a.c1, 160, a.d1, nullptr, B, H1, W1, 1);
-    k_up_fwd<<<blocks(P0 * 64), 256, 0, st>>>(a.d1, a.c0, B, H, W, 64, 96);
-    k_copy_ch<<<blocks(P0 * 32), 256, 0, st>>>(a.s0, 32, 0, a.c0, 96, 64, 32, P0, 0);
-    conv(n, st, D0, a.c0, 96, a.d0, nullptr, B, H, W, 1);
-  } else {  // inference: upsampling and concatenation happen in the convolution's input loader
-    conv_cat(n, st, D2, a.b3, 128, a.s2, 96, a.d2, B, H2, W2);
-    conv_cat(n, st, D1, a.d2, 96, a.s1, 64, a.d1, B, H1, W1);
-    conv_cat(n, st, D0, a.d1, 64, a.s0, 32, a.d0, B, H, W);
-  }
+  // upsampling and concatenation happen in the convolutions' input loaders
+  conv_cat(n, st, D2, a.b3, 128, a.s2, 96, a.d2, B, H2, W2);
+  conv_cat(n, st, D1, a.d2, 96, a.s1, 64, a.d1, B, H1, W1);
+  conv_cat(n, st, D0, a.d1, 64, a.s0, 32, a.d0, B, H, W);
   conv(n, st, HEAD, a.d0, 32, nullptr, a.o, B, H, W, 0);
   ck(cudaGetLastError(), "network forward");
 }
 
-// Backward of layer li: dW += Σ_p dY ⊗ im2col(X), db += Σ_p dY, and (dx != null) dX = conv(dY, flipped W).  dy is the
-// gradient at the layer's pre-activation (already ReLU-masked).
-void conv_bwd(Net& n, cudaStream_t st, int li, const bf16* dy, const bf16* x, int xs, bf16* dx, int B, int H, int W) {
+template <int MT>
+void wgrad_launch_mt(const WgradArgs& a, cudaStream_t st) {
+  using Cfg = WgCfg<MT>;
+  ck(cudaFuncSetAttribute(k_conv_wgrad<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem), "wgrad smem");
+  const long long tiles = (long long)a.B * ((a.H + HT_H - 1) / HT_H) * ((a.W + HT_W - 1) / HT_W);
+  const unsigned gx = (unsigned)((a.cout + Cfg::CO - 1) / Cfg::CO), gy = (unsigned)((a.cin + WG_CI - 1) / WG_CI);
+  // about two CTAs per SM in all, and at least four tiles each: the FP32 reductions into dW cost as much as a tile or two
+  long long z = (2 * 148 + gx * gy - 1) / (gx * gy);
+  z = z < (tiles + 3) / 4 ? z : (tiles + 3) / 4;
+  k_conv_wgrad<MT><<<dim3(gx, gy, (unsigned)z), WG_NT, Cfg::smem, st>>>(a);
+}
+// Output channels per CTA: the largest of 64, 48, 32, 16 that divides cout (16 with padding otherwise).
+void wgrad_launch(const WgradArgs& a, cudaStream_t st) {
+  if (a.cout % 64 == 0) return wgrad_launch_mt<4>(a, st);
+  if (a.cout % 48 == 0) return wgrad_launch_mt<3>(a, st);
+  if (a.cout % 32 == 0) return wgrad_launch_mt<2>(a, st);
+  return wgrad_launch_mt<1>(a, st);
+}
+
+// Backward of layer li: dW += Σ_p dY ⊗ im2col(X), db += Σ_p dY, and (dx != null) dX = conv(dY, flipped W), 0 where
+// `mask` (the ReLU output the layer read) is not positive.  dy is the gradient at the layer's pre-activation.  x2 != null:
+// the layer read the virtual concatenation [up2(x) (xs channels), x2 (x2s channels)].
+void conv_bwd(Net& n, cudaStream_t st, int li, const bf16* dy, const bf16* x, int xs, bf16* dx, const bf16* mask, int B,
+              int H, int W, const bf16* x2 = nullptr, int x2s = 0) {
   const Layer& l = n.L[li];
   const long long P = (long long)B * H * W;
-  WgradArgs wa;
+  WgradArgs wa{};
   wa.dy = dy;
   wa.x = x;
+  wa.x2 = x2;
   wa.dw = n.g + l.off;
   wa.B = B;
   wa.H = H;
   wa.W = W;
   wa.cin = l.cin;
   wa.cin_stride = xs;
-  wa.cin_off = 0;
   wa.cout = l.cout;
-  wa.pix_per_cta = wgrad_chunk(P, 4096);
-  dim3 g((unsigned)((l.cout + CM - 1) / CM), (unsigned)((9 * l.cin + CN - 1) / CN),
-         (unsigned)((P + wa.pix_per_cta - 1) / wa.pix_per_cta));
-  k_conv_wgrad<<<g, 128, 0, st>>>(wa);
-  k_bias_grad<<<256, 256 / l.cout * l.cout, 0, st>>>(dy, n.g + l.off + l.nw(), P, l.cout);
+  wa.split = xs;
+  wa.x2_stride = x2s;
+  wgrad_launch(wa, st);
+  k_bias_grad<<<296, 256, 0, st>>>(dy, n.g + l.off + l.nw(), P, l.cout);
   if (dx) {
     k_flip_weights<<<blocks((long long)l.nw()), 256, 0, st>>>(n.wb + l.off, n.wt, l.cout, l.cin);
     ConvArgs a{};
@@ -1046,56 +1121,36 @@ void conv_bwd(Net& n, cudaStream_t st, int li, const bf16* dy, const bf16* x, in
     a.cin_off = 0;
     a.cout = l.cin;
     a.relu = 0;
+    a.mask = mask;
     conv_launch(a, st);
   }
-}
-
-void relu_bwd(bf16* dy, const bf16* y, long long cnt, cudaStream_t st) {
-  k_relu_bwd<<<blocks(cnt), 256, 0, st>>>(dy, y, cnt);
 }
 
 void backward(Net& n, const Acts& a, int B, int H, int W, cudaStream_t st) {
   const long long P0 = (long long)B * H * W, P1 = P0 / 4, P2 = P0 / 16, P3 = P0 / 64;
   const int H1 = H / 2, W1 = W / 2, H2 = H / 4, W2 = W / 4, H3 = H / 8, W3 = W / 8;
-  conv_bwd(n, st, HEAD, a.g_o, a.d0, 32, a.g_d0, B, H, W);
-  relu_bwd(a.g_d0, a.d0, P0 * 32, st);
-  conv_bwd(n, st, D0, a.g_d0, a.c0, 96, a.g_c0, B, H, W);
-  // c0 = up(d1) ++ s0
-  k_up_bwd<<<blocks(P1 * 64), 256, 0, st>>>(a.g_c0, a.g_d1, B, H, W, 64, 96);
-  k_copy_ch<<<blocks(P0 * 32), 256, 0, st>>>(a.g_c0, 96, 64, a.g_s0, 32, 0, 32, P0, 0);
-  relu_bwd(a.g_d1, a.d1, P1 * 64, st);
-  conv_bwd(n, st, D1, a.g_d1, a.c1, 160, a.g_c1, B, H1, W1);
-  // c1 = up(d2) ++ s1
-  k_up_bwd<<<blocks(P2 * 96), 256, 0, st>>>(a.g_c1, a.g_d2, B, H1, W1, 96, 160);
-  k_copy_ch<<<blocks(P1 * 64), 256, 0, st>>>(a.g_c1, 160, 96, a.g_s1, 64, 0, 64, P1, 0);
-  relu_bwd(a.g_d2, a.d2, P2 * 96, st);
-  conv_bwd(n, st, D2, a.g_d2, a.c2, 224, a.g_c2, B, H2, W2);
-  // c2 = up(b3) ++ s2
-  k_up_bwd<<<blocks(P3 * 128), 256, 0, st>>>(a.g_c2, a.g_b3, B, H2, W2, 128, 224);
-  k_copy_ch<<<blocks(P2 * 96), 256, 0, st>>>(a.g_c2, 224, 128, a.g_s2, 96, 0, 96, P2, 0);
+  conv_bwd(n, st, HEAD, a.g_o, a.d0, 32, a.g_d0, a.d0, B, H, W);
+  conv_bwd(n, st, D0, a.g_d0, a.d1, 64, a.g_c0, nullptr, B, H, W, a.s0, 32);  // up(d1) ++ s0
+  k_up_bwd<<<blocks(P1 * 8), 256, 0, st>>>(a.g_c0, a.d1, a.g_d1, B, H, W, 64, 96);
+  conv_bwd(n, st, D1, a.g_d1, a.d2, 96, a.g_c1, nullptr, B, H1, W1, a.s1, 64);  // up(d2) ++ s1
+  k_up_bwd<<<blocks(P2 * 12), 256, 0, st>>>(a.g_c1, a.d2, a.g_d2, B, H1, W1, 96, 160);
+  conv_bwd(n, st, D2, a.g_d2, a.b3, 128, a.g_c2, nullptr, B, H2, W2, a.s2, 96);  // up(b3) ++ s2
+  k_up_bwd<<<blocks(P3 * 16), 256, 0, st>>>(a.g_c2, a.b3, a.g_b3, B, H2, W2, 128, 224);
   // level 3
-  relu_bwd(a.g_b3, a.b3, P3 * 128, st);
-  conv_bwd(n, st, E3B, a.g_b3, a.a3, 128, a.g_a3, B, H3, W3);
-  relu_bwd(a.g_a3, a.a3, P3 * 128, st);
-  conv_bwd(n, st, E3A, a.g_a3, a.p3, 96, a.g_p3, B, H3, W3);
-  k_pool_bwd<<<blocks(P2 * 96), 256, 0, st>>>(a.g_p3, a.g_s2, B, H2, W2, 96, 1);
+  conv_bwd(n, st, E3B, a.g_b3, a.a3, 128, a.g_a3, a.a3, B, H3, W3);
+  conv_bwd(n, st, E3A, a.g_a3, a.p3, 96, a.g_p3, nullptr, B, H3, W3);
   // level 2
-  relu_bwd(a.g_s2, a.s2, P2 * 96, st);
-  conv_bwd(n, st, E2B, a.g_s2, a.a2, 96, a.g_a2, B, H2, W2);
-  relu_bwd(a.g_a2, a.a2, P2 * 96, st);
-  conv_bwd(n, st, E2A, a.g_a2, a.p2, 64, a.g_p2, B, H2, W2);
-  k_pool_bwd<<<blocks(P1 * 64), 256, 0, st>>>(a.g_p2, a.g_s1, B, H1, W1, 64, 1);
+  k_skip_bwd<<<blocks(P2 * 12), 256, 0, st>>>(a.g_c2, 224, 128, a.g_p3, a.s2, a.g_s2, B, H2, W2, 96);
+  conv_bwd(n, st, E2B, a.g_s2, a.a2, 96, a.g_a2, a.a2, B, H2, W2);
+  conv_bwd(n, st, E2A, a.g_a2, a.p2, 64, a.g_p2, nullptr, B, H2, W2);
   // level 1
-  relu_bwd(a.g_s1, a.s1, P1 * 64, st);
-  conv_bwd(n, st, E1B, a.g_s1, a.a1, 64, a.g_a1, B, H1, W1);
-  relu_bwd(a.g_a1, a.a1, P1 * 64, st);
-  conv_bwd(n, st, E1A, a.g_a1, a.p1, 32, a.g_p1, B, H1, W1);
-  k_pool_bwd<<<blocks(P0 * 32), 256, 0, st>>>(a.g_p1, a.g_s0, B, H, W, 32, 1);
+  k_skip_bwd<<<blocks(P1 * 8), 256, 0, st>>>(a.g_c1, 160, 96, a.g_p2, a.s1, a.g_s1, B, H1, W1, 64);
+  conv_bwd(n, st, E1B, a.g_s1, a.a1, 64, a.g_a1, a.a1, B, H1, W1);
+  conv_bwd(n, st, E1A, a.g_a1, a.p1, 32, a.g_p1, nullptr, B, H1, W1);
   // level 0
-  relu_bwd(a.g_s0, a.s0, P0 * 32, st);
-  conv_bwd(n, st, E0B, a.g_s0, a.a0, 32, a.g_a0, B, H, W);
-  relu_bwd(a.g_a0, a.a0, P0 * 32, st);
-  conv_bwd(n, st, E0A, a.g_a0, a.x, 48, nullptr, B, H, W);
+  k_skip_bwd<<<blocks(P0 * 4), 256, 0, st>>>(a.g_c0, 96, 64, a.g_p1, a.s0, a.g_s0, B, H, W, 32);
+  conv_bwd(n, st, E0B, a.g_s0, a.a0, 32, a.g_a0, a.a0, B, H, W);
+  conv_bwd(n, st, E0A, a.g_a0, a.x, 48, nullptr, nullptr, B, H, W);
   ck(cudaGetLastError(), "network backward");
 }
 
@@ -1336,8 +1391,7 @@ int ps_net_train_step(ps_net* pn, const void* input, const float* labels, uint32
     ck(cudaMemsetAsync(n.stats, 0, 64, st), "cudaMemset");
     ck(cudaMemsetAsync(n.g, 0, n.nparam * 4, st), "cudaMemset");
     k_count_valid<<<blocks(P0), 256, 0, st>>>(labels, P0, n.stats + 2);
-    k_loss<<<blocks(P0), 256, 0, st>>>(a.o, labels, a.g_o, n.stats, P0, 1.f, 1.f / depth_min, 1.f / depth_max);
-    k_scale_grad<<<blocks(P0 * 8), 256, 0, st>>>(a.g_o, P0 * 8, n.stats + 2);
+    k_loss<<<blocks(P0), 256, 0, st>>>(a.o, labels, a.g_o, n.stats, P0, 1.f / depth_min, 1.f / depth_max);
     backward(n, a, B, H, W, st);
     end_use(n, st);
     ck(cudaFreeAsync(a.o, st), "cudaFreeAsync");
@@ -1447,7 +1501,7 @@ int ps_net_conv_check(int device, const uint16_t* x, const float* w, const uint1
     d.cout = (int)cin;
     d.yf = b.dx;
     conv_launch(d, 0);
-    WgradArgs wa;
+    WgradArgs wa{};
     wa.dy = b.dy;
     wa.x = b.x;
     wa.dw = b.dw;
@@ -1456,12 +1510,8 @@ int ps_net_conv_check(int device, const uint16_t* x, const float* w, const uint1
     wa.W = (int)W;
     wa.cin = (int)cin;
     wa.cin_stride = (int)cin;
-    wa.cin_off = 0;
     wa.cout = (int)cout;
-    wa.pix_per_cta = wgrad_chunk(P, 256);
-    dim3 g((unsigned)((cout + CM - 1) / CM), (unsigned)((9 * cin + CN - 1) / CN),
-           (unsigned)((P + wa.pix_per_cta - 1) / wa.pix_per_cta));
-    k_conv_wgrad<<<g, 128>>>(wa);
+    wgrad_launch(wa, 0);
     ck(cudaGetLastError(), "convolution kernels");
     ck(cudaDeviceSynchronize(), "sync");
     ck(cudaMemcpy(y, b.y, P * cout * 4, cudaMemcpyDeviceToHost), "download");

@@ -45,6 +45,22 @@ def test_conv_kernels_match_fp64(shape, path):
     proposal.set_conv_path("auto")
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1, 8, 8), (2, 8, 16, 32, 64), (1, 9, 17, 40, 24), (3, 25, 33, 96, 48),
+                                   (1, 70, 130, 56, 128), (5, 3, 40, 224, 16)])
+def test_weight_gradient_tiles_match_fp64(shape):
+    """The weight gradient at the edges of its 8 x 16 pixel tiles, 32 input and 16/32/48/64 output channel blocks, with
+    one tile and with several per CTA.  Products of bf16 are exact in binary32; each of the P additions rounds once, so
+    the error is at most P * 2^-24 of the sum of magnitudes (twice that is allowed)."""
+    b, h, w, ci, co = shape
+    rng = np.random.default_rng(7 + sum(shape))
+    x, dy = _bf16(rng, (b, h, w, ci)), _bf16(rng, (b, h, w, co))
+    _, _, dw = proposal.conv_check(x, np.zeros((co, 9, ci), np.float32), dy)
+    xf, dyf = O.from_bf16_bits(x), O.from_bf16_bits(dy)
+    _, ref, _ = O.conv_grads(xf, np.zeros((co, 9, ci)), dyf)
+    _, mag, _ = O.conv_grads(np.abs(xf), np.zeros((co, 9, ci)), np.abs(dyf))
+    assert (np.abs(dw - ref) <= b * h * w * 2.0 ** -23 * mag + 1e-30).all()
+
+
 def _labels(rng, b, h, w, dr=(25.0, 60.0)):
     lab = np.zeros((b, h, w, 6), np.float32)
     lab[..., 0] = rng.uniform(0, 1, (b, h, w))
