@@ -19,9 +19,10 @@ struct SpkArgs {
   const float* cost;   // final matching costs
   int* parent;         // union-find parent per slot pixel (-1 = invalid)
   int* size;           // component size per root
-  unsigned* lo;        // bisection bounds per small root (order-preserving cost keys)
-  unsigned* hi;
-  unsigned* cnt;
+  unsigned* lo;        // small components: start of their run of cost keys, per root
+  unsigned* hi;        // the runs: order-preserving cost keys, at most one per pixel
+  unsigned* cnt;       // keys placed per root, then its median key
+  unsigned* nkeys;     // keys in all runs (device counter)
   unsigned long long* removed;
   unsigned long long* valid;  // k_count_valid: valid pixels of the items
   float rel, keep;

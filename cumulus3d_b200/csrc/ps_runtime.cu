@@ -2010,7 +2010,7 @@ int ps_propose(ps_session* s, ps_net* net, uint32_t level, const uint32_t* views
     }
     grow(s, s->netin, s->netin_cap, in_need);
     grow(s, s->netout, s->netout_cap, out_need);
-    if (!s->pcount) s->pcount = dalloc<unsigned long long>(s, 2);  // two counters (post-processing uses both)
+    if (!s->pcount) s->pcount = dalloc<unsigned long long>(s, 3);  // two counters (post-processing uses both)
     cuda_ok(cudaMemsetAsync(s->pcount, 0, sizeof(unsigned long long), s->st), "memset");
     for (size_t i = 0; i < n; ++i) {
       const uint32_t v = views[i];
@@ -2188,7 +2188,7 @@ int ps_postprocess_resident(ps_session* s, uint32_t level, const uint32_t* views
     if (filled) *filled = 0;
     if (n == 0 || (!p->remove_speckles && !p->fill_holes)) return;
     if (!sl.spk) sl.spk = dalloc<int>(s, (size_t)std::max<long long>(sl.total, 1) * 5);
-    if (!s->pcount) s->pcount = dalloc<unsigned long long>(s, 2);
+    if (!s->pcount) s->pcount = dalloc<unsigned long long>(s, 3);
     cuda_ok(cudaMemsetAsync(s->pcount, 0, 2 * sizeof(unsigned long long), s->st), "memset");
     const size_t T = (size_t)std::max<long long>(sl.total, 1);
     if (p->remove_speckles)
@@ -2203,6 +2203,7 @@ int ps_postprocess_resident(ps_session* s, uint32_t level, const uint32_t* views
       A.hi = (unsigned*)(sl.spk + 3 * T);
       A.cnt = (unsigned*)(sl.spk + 4 * T);
       A.removed = s->pcount;
+      A.nkeys = reinterpret_cast<unsigned*>(s->pcount + 2);
       A.rel = p->speckle_rel_depth;
       A.keep = p->speckle_keep_cost;
       const int tiles = spk_items(s, A, views, a, b, (int)level, p->speckle_min_area_frac);
