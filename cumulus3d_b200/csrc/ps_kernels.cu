@@ -163,7 +163,7 @@ __device__ __forceinline__ float src_sample(unsigned long long tex, float u, flo
 
 // ------------------------------------------------------------------------------------------- reference window
 struct RefStats {
-  float ic, W, mu, var;
+  float ic, W, iW, mu, var;  // iW = 1 / W
 };
 
 // Tile-resident reference window of one pixel: t points at the pixel inside the shared tile (row pitch tw).  Window sums
@@ -245,6 +245,7 @@ __device__ __forceinline__ RefStats ref_stats(const PsRun& P, const RefWin& rw) 
   }
   s.W = W[0] + W[1];
   const float St = S[0] + S[1], SSt = SS[0] + SS[1];
+  s.iW = 1.0f / s.W;
   s.mu = St / s.W;
   s.var = SSt / s.W - s.mu * s.mu;
   return s;
@@ -289,7 +290,7 @@ __device__ __forceinline__ bool ncc_begin(const RefStats& rs, const PsLevel& S, 
 }
 // Epilogue (patchmatch.cu:280-289) from the window totals.
 __device__ __forceinline__ float ncc_finish(const RefStats& rs, float Sst, float SSst, float ISt) {
-  float iW = 1.0f / rs.W;
+  const float iW = rs.iW;
   float mus = Sst * iW;
   float vars = SSst * iW - mus * mus;
   if (vars < 1e-5f) return 2.0f;
@@ -672,10 +673,10 @@ __device__ __forceinline__ float ncc_cost_warp(const PsRun& P, const RefWin& rw,
 // Forward/backward reprojection error through the source snapshot (patchmatch.cu:292-314); INF on failure.
 #define PS_INF_ERR 1e30f
 __device__ float geo_error(const PsRun& P, const PsLevel& R, const PsLevel& S, const PsPair& pr, int x, int y,
-                           float d) {
+                           float3 ray, float d) {
   long long off = P.snap_off[pr.src];
   if (off < 0) return PS_INF_ERR;
-  float3 X = make_float3(((float)x - R.cx) / R.fx * d, ((float)y - R.cy) / R.fy * d, d);
+  float3 X = make_float3(ray.x * d, ray.y * d, d);  // ray = pixel_ray(R, x, y)
   float xj = pr.r[0] * X.x + pr.r[1] * X.y + pr.r[2] * X.z + pr.t[0];
   float yj = pr.r[3] * X.x + pr.r[4] * X.y + pr.r[5] * X.z + pr.t[1];
   float zj = pr.r[6] * X.x + pr.r[7] * X.y + pr.r[8] * X.z + pr.t[2];
@@ -704,7 +705,7 @@ __device__ __forceinline__ float pair_cost(const PsRun& P, const RefWin& rw, con
   float H[9];
   float c = 2.0f;
   if (homography(R, lp, (float)x, (float)y, h, H)) c = ncc_cost<WR, WS, CW, NT>(P, rw, rs, S, H, x, y, nwin);
-  if (P.geometric) *geo = fminf(geo_error(P, R, S, pr, x, y, h.w), P.gmax);
+  if (P.geometric) *geo = fminf(geo_error(P, R, S, pr, x, y, pixel_ray(R, x, y), h.w), P.gmax);
   return c;
 }
 
@@ -884,13 +885,15 @@ __device__ __forceinline__ void propagation_candidates(const PsLevel& R, const f
 
 // 2. View selection and aggregation (patchmatch.cu:513-594): per source, votes over the 8 propagated hypotheses,
 // the view weight, and the weighted cost sums of the 9 hypotheses; then the aggregated argmin.
+// (The loops over the 9 hypotheses are rolled: the arrays then live in local memory, not in registers that the window loops
+// need.)
 struct ViewAgg {
   float num[9], numf[9];
   float den, denf, wbest;
   int vbest;
 };
 __device__ __forceinline__ void agg_init(ViewAgg& a) {
-#pragma unroll
+#pragma unroll 1
   for (int i = 0; i < 9; ++i) {
     a.num[i] = 0.f;
     a.numf[i] = 0.f;
@@ -917,7 +920,7 @@ __device__ __forceinline__ void agg_source(const PsRun& P, float tau_good, ViewA
                                            float prior, int j, int vprev, float* wvj) {
   int good = 0, bad = 0;
   float conf = 0.f;
-#pragma unroll
+#pragma unroll 1
   for (int i = 1; i < 9; ++i) {
     if (m[i] < tau_good) {
       good++;
@@ -930,11 +933,11 @@ __device__ __forceinline__ void agg_source(const PsRun& P, float tau_good, ViewA
   const float wp = adopt ? (isprev ? 2.f : 1.f) * conf / (float)good : (isprev ? P.prev_w : 0.f);
   const float w2 = wp * prior;
   *wvj = w2 > 0.f ? w2 : -prior;
-#pragma unroll
+#pragma unroll 1
   for (int i = 0; i < 9; ++i) a.numf[i] += prior * (m[i] + P.lambda * gg[i]);
   a.denf += prior;
   if (w2 > 0.f) {
-#pragma unroll
+#pragma unroll 1
     for (int i = 0; i < 9; ++i) a.num[i] += w2 * (m[i] + P.lambda * gg[i]);
     a.den += w2;
     if (w2 > a.wbest) {
@@ -950,26 +953,26 @@ __device__ __forceinline__ void agg_finish(ViewAgg& a, const float4* hyp, int ns
   float agg[9];
   int bi9 = 0;
   if (a.den > 0.f) {
-#pragma unroll
+#pragma unroll 1
     for (int i = 0; i < 9; ++i) agg[i] = a.num[i] / a.den;
   } else if (a.denf > 0.f) {
-#pragma unroll
+#pragma unroll 1
     for (int i = 0; i < 9; ++i) agg[i] = a.numf[i] / a.denf;
     for (int j = 0; j < nsrc; ++j) wv[j * wstride] = -wv[j * wstride];
     a.den = a.denf;
   } else {
-#pragma unroll
+#pragma unroll 1
     for (int i = 0; i < 9; ++i) agg[i] = 2.f;
   }
   float bagg = agg[0];
-#pragma unroll
+#pragma unroll 1
   for (int i = 1; i < 9; ++i)
     if (agg[i] < bagg) {
       bagg = agg[i];
       bi9 = i;
     }
   best = hyp[0];
-#pragma unroll
+#pragma unroll 1
   for (int i = 1; i < 9; ++i)
     if (i == bi9) best = hyp[i];
   bcost = bagg;
@@ -1110,13 +1113,8 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
       float H[9];
       const bool ok = homography(R, lp, (float)x, (float)y, hyp[i], H);
       const float mi = window(S, H, ok);
-      const float gi = P.geometric ? fminf(geo_error(P, R, S, pr, x, y, hyp[i].w), P.gmax) : 0.f;
-#pragma unroll
-      for (int q = 0; q < 9; ++q)
-        if (q == i) {
-          m[q] = mi;
-          gg[q] = gi;
-        }
+      m[i] = mi;
+      gg[i] = P.geometric ? fminf(geo_error(P, R, S, pr, x, y, ray, hyp[i].w), P.gmax) : 0.f;
     }
     agg_source(P, ph.tau_good, ag, m, gg, prior, j, vprev, wv + j * NT);
   }
@@ -1129,6 +1127,14 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
   // round-to-nearest addition and division by den > 0 are monotone), so once the partial cost reaches bcost the
   // candidate cannot be adopted (the test is cc < bcost) and its remaining windows are skipped: same decisions,
   // same bits.
+  //
+  // Geometric runs know part of the sources still to come before any window: their terms are at least wj·λ·g.  Their sum
+  // (rem) joins the test, less 1e-5 of it for the rounding of taking the terms out again and 1e-4 of the whole, which is
+  // far above what rounding can take from at most 32 added terms (32·2^-22).  A candidate at a random depth is mostly
+  // beaten by it without a window, and those windows are the dearest: their lanes gather from unrelated places (5 views
+  // of 1920 × 1080, 2 photometric and 1 geometric iterations: 415 -> 399 ms for the whole schedule).
+  const bool bound = P.geometric && P.lambda > 0.f;
+  float gs[PS_MAXSRC];
   Refine rf;
   int nskip = 0;
   refine_prior(P, base + pix, rs.var, ray, rf);
@@ -1138,13 +1144,24 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
     const float4 cd = refine_candidate(rf, c);
     float cc;
     if (ag.den > 0.f) {
-      float nm = 0.f;
+      float nm = 0.f, rem = 0.f;
       bool beaten = false;
+      if (bound) {
+#pragma unroll 1
+        for (int j = 0; j < nsrc; ++j) {
+          const float wj = wv[j * NT];
+          if (!(wj > 0.f)) continue;
+          const PsLevel& S = P.lv[prs[j].src * P.nlevels + P.level];
+          gs[j] = fminf(geo_error(P, R, S, prs[j], x, y, ray, cd.w), P.gmax);
+          rem += wj * (P.lambda * gs[j]);
+        }
+      }
+      const float slack = 1e-5f * rem;
 #pragma unroll 1
       for (int j = 0; j < nsrc; ++j) {  // no break: the warp's lanes keep stepping through the sources together
         const float wj = wv[j * NT];
         if (!(wj > 0.f)) continue;
-        beaten = beaten || nm / ag.den >= bcost;
+        beaten = beaten || nm / ag.den >= bcost || (bound && 0.9999f * (nm + (rem - slack)) / ag.den >= bcost);
         if (beaten) {
           nskip++;
           continue;
@@ -1155,8 +1172,9 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
         float H[9];
         const bool hok = homography(R, lp, (float)x, (float)y, cd, H);
         const float mm = window(S, H, hok);
-        const float g = P.geometric ? fminf(geo_error(P, R, S, pr, x, y, cd.w), P.gmax) : 0.f;
+        const float g = bound ? gs[j] : P.geometric ? fminf(geo_error(P, R, S, pr, x, y, ray, cd.w), P.gmax) : 0.f;
         nm += wj * (mm + P.lambda * g);
+        rem -= bound ? wj * (P.lambda * g) : 0.f;
       }
       cc = beaten ? bcost : nm / ag.den;
     } else {
@@ -1409,7 +1427,7 @@ __global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_st(const __grid_constant
       mv = ncc_cost_warp<WR, WS, NT, TMA>(P, rw, rs, S, pr.src, H, x, y, act && hok, nwin, box, bs);
     }
     if (trav) {
-      const float gv = (P.geometric && use) ? fminf(geo_error(P, R, S, pr, x, y, hv.w), P.gmax) : 0.f;
+      const float gv = (P.geometric && use) ? fminf(geo_error(P, R, S, pr, x, y, ray, hv.w), P.gmax) : 0.f;
 #pragma unroll
       for (int q = 0; q < 9; ++q)
         if (q == i) {
@@ -1419,7 +1437,7 @@ __global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_st(const __grid_constant
       if (i == 8 && use) agg_source(P, ph.tau_good, ag, m, gg, prior, j, vprev, wv + j * NT);
     } else {
       if (act) {
-        const float g = P.geometric ? fminf(geo_error(P, R, S, pr, x, y, hv.w), P.gmax) : 0.f;
+        const float g = P.geometric ? fminf(geo_error(P, R, S, pr, x, y, ray, hv.w), P.gmax) : 0.f;
         nm += wj * (mv + P.lambda * g);
       }
       if (j == nsrc - 1) {
@@ -1677,7 +1695,7 @@ __global__ void __launch_bounds__(PS_EVAL_NT, half_min_ctas(WR, WS)) k_filter(co
       const float m = ncc_cost<WR, WS, CW, NT>(P, rw, rs, S, H, x, y, nwin);
       const float ee = P.ncc_norm * m_exp(-m * m * P.inv2ncc);
       if (ee / (ee + 0.5f) < P.q_min) continue;
-      if (geo_error(P, e.R, S, pr, x, y, h.w) > P.filter_gmax) continue;
+      if (geo_error(P, e.R, S, pr, x, y, ray, h.w) > P.filter_gmax) continue;
       count++;
     }
   }
