@@ -949,9 +949,9 @@ __device__ __forceinline__ void agg_source(const PsRun& P, float tau_good, ViewA
 // Aggregated costs, the prior-weighted fallback (view weights become the priors, den = denf), the argmin (earliest on
 // ties); returns the best hypothesis and its cost.
 __device__ __forceinline__ void agg_finish(ViewAgg& a, const float4* hyp, int nsrc, float* wv, int wstride,
-                                           float4& best, float& bcost) {
+                                           float4& best, float& bcost, int& bi9) {
   float agg[9];
-  int bi9 = 0;
+  bi9 = 0;
   if (a.den > 0.f) {
 #pragma unroll 1
     for (int i = 0; i < 9; ++i) agg[i] = a.num[i] / a.den;
@@ -1091,7 +1091,16 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
   };
 
   // 2. View traversal: voting, weighting, aggregation.
+  //
+  // The current plane (hypothesis 0) was matched before: by the run start against every source, or by this pixel's last
+  // half step, as one of its hypotheses or as an adopted candidate.  Its costs of then are kept (the same window of the
+  // same plane has the same bits), and only a source not known from then runs its window again.
   const int vprev = P.bview[base + pix];
+  const int nkeep = min(nsrc, P.keep);
+  float* const kept = P.kept + base + pix;
+  const float unknown = __int_as_float(0x7fffffff);
+  float mall[9 * (PS_KEEP + 1)], mbest[PS_KEEP], mcand[PS_KEEP];
+  unsigned seen = 0u;
   ViewAgg ag;
   agg_init(ag);
 #pragma unroll 1
@@ -1099,7 +1108,8 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
     const PsPair& pr = prs[j];
     const PsLPair lp = lps[j];
     const PsLevel S = P.lv[pr.src * P.nlevels + P.level];
-    float m[9], gg[9];
+    float* const m = mall + 9 * min(j, PS_KEEP);
+    float gg[9];
     float prior;
     wv[j * NT] = 0.f;
     {
@@ -1108,11 +1118,16 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
       prior = view_prior(P, R, pr, H, ok, x, y, hyp[0], wr);
       if (!(prior > 0.f)) continue;
     }
+    const float m0 = j < nkeep ? kept[j * P.keep_stride] : unknown;
+    seen |= j < nkeep ? 1u << j : 0u;
 #pragma unroll 1
     for (int i = 0; i < 9; ++i) {
-      float H[9];
-      const bool ok = homography(R, lp, (float)x, (float)y, hyp[i], H);
-      const float mi = window(S, H, ok);
+      float mi = m0;
+      if (i > 0 || !(m0 == m0)) {
+        float H[9];
+        const bool ok = homography(R, lp, (float)x, (float)y, hyp[i], H);
+        mi = window(S, H, ok);
+      }
       m[i] = mi;
       gg[i] = P.geometric ? fminf(geo_error(P, R, S, pr, x, y, ray, hyp[i].w), P.gmax) : 0.f;
     }
@@ -1120,7 +1135,14 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
   }
   float4 best;
   float bcost;
-  agg_finish(ag, hyp, nsrc, wv, NT, best, bcost);
+  int bi;
+  agg_finish(ag, hyp, nsrc, wv, NT, best, bcost, bi);
+#pragma unroll 1
+  for (int j = 0; j < nkeep; ++j)
+    mbest[j] = !(hyp[bi].w > 0.f)  ? unknown  // refine_draw gives such a plane another depth
+               : (seen >> j & 1u)  ? mall[9 * j + bi]
+               : bi == 0           ? kept[j * P.keep_stride]
+                                   : unknown;
 
   // 3. Refinement, 6 hypotheses (patchmatch.cu:596-628), then 4. the coarse-scale candidate (:629-653).
   // A candidate's cost nm / den only grows as sources are added (every term wj·(mm + λ·g) is finite and ≥ 0, and
@@ -1146,6 +1168,8 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
     if (ag.den > 0.f) {
       float nm = 0.f, rem = 0.f;
       bool beaten = false;
+#pragma unroll 1
+      for (int j = 0; j < nkeep; ++j) mcand[j] = unknown;
       if (bound) {
 #pragma unroll 1
         for (int j = 0; j < nsrc; ++j) {
@@ -1172,6 +1196,7 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
         float H[9];
         const bool hok = homography(R, lp, (float)x, (float)y, cd, H);
         const float mm = window(S, H, hok);
+        if (j < nkeep) mcand[j] = mm;
         const float g = bound ? gs[j] : P.geometric ? fminf(geo_error(P, R, S, pr, x, y, ray, cd.w), P.gmax) : 0.f;
         nm += wj * (mm + P.lambda * g);
         rem -= bound ? wj * (P.lambda * g) : 0.f;
@@ -1183,8 +1208,12 @@ __device__ __forceinline__ void half_tile(const PsRun& P, const HalfPhase& ph, i
     if (cc < bcost) {
       bcost = cc;
       best = cd;
+#pragma unroll 1
+      for (int j = 0; j < nkeep; ++j) mbest[j] = ag.den > 0.f ? mcand[j] : unknown;
     }
   }
+#pragma unroll 1
+  for (int j = 0; j < nkeep; ++j) kept[j * P.keep_stride] = mbest[j];
   pl[pix] = best;
   P.cost[base + pix] = bcost;
   P.bview[base + pix] = (unsigned char)ag.vbest;
@@ -1381,7 +1410,8 @@ __global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_st(const __grid_constant
 #pragma unroll 1
   for (int k = 0;; ++k) {
     if (k == nA) {  // end of the traversal: aggregate, then the refinement draws
-      agg_finish(ag, hyp, nsrc, wv, NT, best, bcost);
+      int bi;
+      agg_finish(ag, hyp, nsrc, wv, NT, best, bcost, bi);
       refine_draw(P, ph, vd, pix, ray, best, rf);
     }
     if (k == nA + nB) break;
@@ -1476,7 +1506,7 @@ __global__ void __launch_bounds__(PS_HALF_NT, 2) k_half_st(const __grid_constant
 // Top-K mean cost (patchmatch.cu:327-345).
 template <int WR, int WS, bool CW, int NT>
 __device__ float topk_cost(const PsRun& P, const RefWin& rw, const RefStats& rs, const PsLevel& R, const PsPair* prs,
-                           const PsLPair* lps, int nsrc, int x, int y, float4 h, int& nwin) {
+                           const PsLPair* lps, int nsrc, int x, int y, float4 h, float* kept, int& nwin) {
   float b0 = 1e30f, b1 = 1e30f, b2 = 1e30f;
 #pragma unroll 1
   for (int j = 0; j < nsrc; ++j) {
@@ -1485,6 +1515,7 @@ __device__ float topk_cost(const PsRun& P, const RefWin& rw, const RefStats& rs,
     const PsLevel S = P.lv[pr.src * P.nlevels + P.level];
     float g = 0.f;
     float c = pair_cost<WR, WS, CW, NT>(P, rw, rs, R, S, pr, lp, x, y, h, &g, nwin);
+    if (kept && j < P.keep) kept[j * P.keep_stride] = c;
     if (P.geometric) c += P.lambda * g;
     if (c < b0) {
       b2 = b1;
@@ -1574,9 +1605,12 @@ __global__ void __launch_bounds__(PS_EVAL_NT, half_min_ctas(WR, WS)) k_eval(cons
   }
   float c = 2.f;
   int nwin = 0;
+  float* const kept = P.mode == 1 && P.keep > 0 ? P.kept + base + pix : nullptr;  // run start: for its half steps
   if (h.w > 0.f) {
     const RefStats rs = ref_stats<WR, WS, CW, NT>(P, rw);
-    c = topk_cost<WR, WS, CW, NT>(P, rw, rs, e.R, prs, lps, vd.nsrc, x, y, h, nwin);
+    c = topk_cost<WR, WS, CW, NT>(P, rw, rs, e.R, prs, lps, vd.nsrc, x, y, h, kept, nwin);
+  } else if (kept) {
+    for (int j = 0; j < min(vd.nsrc, P.keep); ++j) kept[j * P.keep_stride] = __int_as_float(0x7fffffff);
   }
   P.cost[base + pix] = c;
   if (P.mode == 1) P.bview[base + pix] = 255;

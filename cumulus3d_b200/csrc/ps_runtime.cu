@@ -96,6 +96,8 @@ struct Slot {
   float4* aux = nullptr;    // second plane buffer (median input, readout output)
   float4* prior = nullptr;  // coarse-scale candidates
   float* cost = nullptr;
+  float* kept = nullptr;    // costs of the current planes within a run (PsRun::kept), `keep` per pixel
+  int keep = 0;
   unsigned char* bview = nullptr;
   unsigned char* count = nullptr;
   std::vector<char> prior_valid;
@@ -397,6 +399,17 @@ Slot& slot(ps_session* s, int level) {
     sl.aux = dalloc<float4>(s, tot);
     sl.prior = dalloc<float4>(s, tot);
     sl.cost = dalloc<float>(s, tot);
+    {  // the kept costs only save work: without memory for them the run does without
+      const int most = s->nsrc.empty() ? 0 : *std::max_element(s->nsrc.begin(), s->nsrc.end());
+      void* k = nullptr;
+      sl.keep = std::min(most, PS_KEEP);
+      const size_t bytes = (size_t)std::max<long long>(tot, 1) * sl.keep * sizeof(float);
+      if (sl.keep > 0 && s->be && s->be->pool && cudaMallocFromPoolAsync(&k, bytes, s->be->pool, s->st) != cudaSuccess) {
+        cudaGetLastError();
+        k = nullptr;
+      }
+      sl.kept = (float*)k;
+    }
     sl.bview = dalloc<unsigned char>(s, tot);
     sl.count = dalloc<unsigned char>(s, tot);
     cuda_ok(cudaMemsetAsync(sl.plane, 0, std::max<long long>(tot, 1) * sizeof(float4), s->st), "memset");
@@ -477,6 +490,9 @@ PsRun base_params(ps_session* s, int level) {
   Slot& sl = slot(s, level);
   P.plane = sl.plane;
   P.cost = sl.cost;
+  P.kept = sl.kept;
+  P.keep_stride = sl.total;
+  P.keep = sl.kept ? sl.keep : 0;
   P.bview = sl.bview;
   P.count = sl.count;
   P.prior = sl.prior;
@@ -1179,6 +1195,7 @@ int ps_end(ps_session* s) {
     dfree(s, sl.aux);
     dfree(s, sl.prior);
     dfree(s, sl.cost);
+    dfree(s, sl.kept);
     dfree(s, sl.bview);
     dfree(s, sl.count);
     dfree(s, sl.proposal);

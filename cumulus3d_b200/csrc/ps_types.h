@@ -21,6 +21,7 @@
 // Reference tile pitch of the staged half step (≡ 4 mod 8: the warp's 8 × 8 block reads it without bank conflicts).
 #define PS_HALF_ST_TW(wr) ((((PS_HALF_PW) + 2 * (wr) + 3) / 8) * 8 + 4)
 #define PS_STAGE_MIN_LANES 4
+#define PS_KEEP 8  // sources whose costs of the current plane a run keeps
 #define PS_STAGE_STATS 8  // profiling counters of the staged half step per kernel kind
 // Evaluate / filter CTA: 128 threads covering 32 × 4 pixels (a warp is one row).
 #define PS_EVAL_NT 128
@@ -119,6 +120,11 @@ struct PsRun {
   int t, color, random_init, topk;
   int use_prior, nitems, ntiles, maxsrc;
   int wr, ws;  // runtime window for the generic kernels
+  // Matching costs of every pixel's current plane against its view's first `keep` sources (NaN: not known), source after
+  // source `keep_stride` pixels apart; written by the run start, kept up by the run's half steps.  Null: none are kept.
+  float* kept;
+  long long keep_stride;
+  int keep, pad0;
   float tau_good, tau_bad, inv2beta2, prev_w;
   int n1, n2;
   float inv2s, inv2c;
