@@ -210,11 +210,13 @@ __global__ void k_spk_median(SpkArgs A) {
     const int src = __ffs(m) - 1;
     const int len = __shfl_sync(0xffffffffu, n, src);
     const unsigned* run = A.hi + __shfl_sync(0xffffffffu, at, src);
-    unsigned lo = 0u, hi = 0xFFFFFFFFu;
+    unsigned key[4], lo = 0u, hi = 0xFFFFFFFFu;  // the first 128 keys in registers
+#pragma unroll
+    for (int k = 0; k < 4; ++k) key[k] = (int)threadIdx.x + 32 * k < len ? run[threadIdx.x + 32 * k] : 0xFFFFFFFFu;
     for (int it = 0; it < 32; ++it) {
-      const unsigned mid = lo + (hi - lo) / 2u;
-      int c = 0;
-      for (int k = threadIdx.x; k < len; k += 32) c += run[k] <= mid;
+      const unsigned mid = lo + (hi - lo) / 2u;  // below 0xFFFFFFFF: the missing keys never count
+      int c = (key[0] <= mid) + (key[1] <= mid) + (key[2] <= mid) + (key[3] <= mid);
+      for (int k = 128 + threadIdx.x; k < len; k += 32) c += run[k] <= mid;
       c = __reduce_add_sync(0xffffffffu, c);
       if (c >= len / 2 + 1) hi = mid;
       else lo = mid + 1u;
@@ -409,15 +411,11 @@ __device__ void fuse_emit(const FuseArgs& A, const FuseView& cv, int v, int col,
   A.nvis[slot] = (unsigned char)write_vis(A.vis + slot * A.vis_stride, v, hits, nh);
 }
 
-// First pass (fusion.rs:243-333) of view A.v: one thread per reference pixel.
-__global__ void __launch_bounds__(256) k_fuse(FuseArgs A) {
-  const FuseView& cv = A.views[A.v];
-  const int col = blockIdx.x * 32 + threadIdx.x, row = blockIdx.y * 8 + threadIdx.y;
-  if (col >= cv.w || row >= cv.h) return;
+// First pass (fusion.rs:243-333) of view A.v.  A CTA takes a 32 × 32 tile: its pixels with depth that no earlier view used
+// go into a list first (after the first views they are few and scattered), and one thread evaluates each of the list.
+__device__ void fuse_pixel(const FuseArgs& A, const FuseView& cv, int col, int row) {
   const long long pix = (long long)row * cv.w + col;
   const float4 q = A.plane[cv.off + pix];
-  if (!(q.w > 0.0f)) return;
-  if (A.mark_used && A.marks[cv.off + pix] != 0) return;
   Hit hits[PS_FUSE_MAX_OVERLAP];
   int nh;
   FusePoint P;
@@ -446,6 +444,30 @@ __global__ void __launch_bounds__(256) k_fuse(FuseArgs A) {
     for (int i = 0; i < nh; ++i) A.consumed[A.views[hits[i].o].off + hits[i].q] = 1;
   }
   fuse_emit(A, cv, A.v, col, row, P, hits, nh);
+}
+
+__global__ void __launch_bounds__(256) k_fuse(FuseArgs A) {
+  __shared__ unsigned short list[1024];
+  __shared__ int count;
+  const FuseView& cv = A.views[A.v];
+  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, tid = threadIdx.y * 32 + threadIdx.x;
+  if (tid == 0) count = 0;
+  __syncthreads();
+  for (int ty = threadIdx.y; ty < 32; ty += 8) {
+    const int col = x0 + threadIdx.x, row = y0 + ty;
+    bool todo = false;
+    if (col < cv.w && row < cv.h) {
+      const long long g = cv.off + (long long)row * cv.w + col;
+      todo = A.plane[g].w > 0.0f && !(A.mark_used && A.marks[g] != 0);
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, todo);
+    int at = 0;
+    if (threadIdx.x == 0 && m) at = atomicAdd(&count, __popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(m & ((1u << threadIdx.x) - 1u));
+    if (todo) list[at] = (unsigned short)(ty * 32 + threadIdx.x);
+  }
+  __syncthreads();
+  for (int i = tid; i < count; i += 256) fuse_pixel(A, cv, x0 + (list[i] & 31), y0 + (list[i] >> 5));
 }
 
 // ---- second pass of leftover pixels (fusion.rs:540-627) ------------------------------------------------------
@@ -984,7 +1006,7 @@ cudaError_t launch_smooth_pass(const SmoothArgs& A, cudaStream_t st) {
 }
 
 cudaError_t launch_fuse(const FuseArgs& A, int w, int h, cudaStream_t st) {
-  const dim3 b(32, 8), g((w + 31) / 32, (h + 7) / 8);
+  const dim3 b(32, 8), g((w + 31) / 32, (h + 31) / 32);
   k_fuse<<<g, b, 0, st>>>(A);
   return cudaGetLastError();
 }

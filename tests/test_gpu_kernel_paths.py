@@ -1,0 +1,110 @@
+"""Device paths at the sizes where they can go wrong, against the CPU oracle bit for bit: windows without a kernel of their
+own, the costs a run keeps (more sources than it keeps, planes without depth), the speckle tiles' edges, the median's."""
+import numpy as np
+import pytest
+
+from cumulus3d_b200 import fusion, scenes
+from cumulus3d_b200.patchstereo import DepthSnapshot, PatchMatchBackend, RunParams, ViewState
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(a, b, what):
+    for k in ("depth", "normal", "cost"):
+        np.testing.assert_array_equal(getattr(a, k), getattr(b, k), err_msg=f"{what} {k}")
+
+
+def _new(wl):
+    return [ViewState.new(c.width, c.height) for c in wl.cams]
+
+
+@pytest.mark.parametrize("wr,ws", [(1, 1), (2, 2), (4, 1), (6, 2), (7, 1), (7, 2), (10, 1)])
+def test_uncompiled_windows_default_tuning(wr, ws):
+    """Even and odd row and column counts, four and eight columns unrolled, with and without the weight cache; an image
+    side below a tile and one above it."""
+    wl = scenes.workload_small(67, 13, views=3, window_radius=wr, window_step=ws, seed=40 + wr)
+    gpu, cpu = _new(wl), _new(wl)
+    p1, p2 = RunParams(0, False, True, 2, 1), RunParams(0, True, False, 1, 2)
+    be = PatchMatchBackend(0)
+    with be.begin(wl.input) as s:
+        s.run(wl.views, gpu, p1)
+        oracle.run(wl.input, wl.views, cpu, p1)
+        snap = DepthSnapshot(1, 0, [g.depth.copy() for g in gpu])
+        s.run(wl.views, gpu, p2, snap)
+        oracle.run(wl.input, wl.views, cpu, p2, snap)
+    be.close()
+    for a, b in zip(gpu, cpu):
+        _same(a, b, f"window {wr},{ws}")
+
+
+@pytest.mark.parametrize("tuning", [0, 42])
+@pytest.mark.parametrize("sources", [1, 8, 11])
+def test_kept_costs_over_runs(sources, tuning):
+    """Three iterations, then a run on other planes (some without depth) of the same session, then a geometric one: the
+    costs kept for the first 8 sources never outlive their plane or their run."""
+    wl = scenes.workload_small(56, 40, views=12, window_radius=3, seed=61, sources=sources, positions=4)
+    rng = np.random.default_rng(5)
+    gpu, cpu = _new(wl), _new(wl)
+    be = PatchMatchBackend(0, tuning=tuning)
+    with be.begin(wl.input) as s:
+        p = RunParams(0, False, True, 3, 1)
+        s.run(wl.views, gpu, p)
+        oracle.run(wl.input, wl.views, cpu, p)
+        for a, b in zip(gpu, cpu):
+            _same(a, b, "first run")
+        for st in gpu:
+            st.depth[...] = np.where(rng.random(st.depth.shape) < 0.2, 0.0, st.depth * rng.uniform(0.8, 1.3, st.depth.shape))
+        cpu = [g.copy() for g in gpu]
+        p = RunParams(0, False, False, 2, 2)
+        s.run(wl.views, gpu, p)
+        oracle.run(wl.input, wl.views, cpu, p)
+        snap = DepthSnapshot(1, 0, [g.depth.copy() for g in gpu])
+        p = RunParams(0, True, False, 2, 3)
+        s.run(wl.views, gpu, p, snap)
+        oracle.run(wl.input, wl.views, cpu, p, snap)
+    be.close()
+    for a, b in zip(gpu, cpu):
+        _same(a, b, f"{sources} sources")
+
+
+@pytest.mark.parametrize("w,h,frac", [(31, 7, 0.05), (32, 8, 0.1), (33, 9, 0.05), (96, 65, 0.002), (130, 70, 0.03)])
+def test_speckles_at_tile_edges(w, h, frac):
+    """Components inside, along and across the 32 x 8 tiles of one-iteration maps (many of them), with limits up to more
+    than 128 pixels."""
+    wl = scenes.workload_small(w, h, views=3, window_radius=3, seed=w + h)
+    post = fusion.default_post()
+    post.speckle_min_area_frac = frac
+    be = PatchMatchBackend(0)
+    with be.begin(wl.input) as s:
+        s.schedule_resident(wl.views, 1, 0, 0)
+        before = s.readout_resident(wl.views)
+        removed = s.postprocess_resident(0, wl.views, post)
+        after = s.readout_download(0, wl.views)
+    be.close()
+    n = 0
+    for b, a in zip(before, after):
+        d, nn = b.depth.copy(), b.normal.copy()
+        n += oracle.remove_speckles(d, nn, b.cost, post)
+        np.testing.assert_array_equal(a.depth, d)
+        np.testing.assert_array_equal(a.normal, nn)
+    assert removed == n
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (2, 5), (33, 9)])
+def test_median_at_edges_and_ties(w, h):
+    wl = scenes.workload_small(w, h, views=2, window_radius=1, seed=3, sources=1)
+    rng = np.random.default_rng(w + h)
+    states = []
+    for c in wl.cams:
+        st = ViewState.new(w, h)
+        st.depth[...] = np.where(rng.random((h, w)) < 0.2, 0.0, rng.integers(28, 32, (h, w)))
+        st.normal[..., 2] = -1.0
+        states.append(st)
+    be = PatchMatchBackend(0)
+    with be.begin(wl.input) as s:
+        got = s.median_filter(wl.input, 0, wl.views, states)
+    be.close()
+    for a, b in zip(got, oracle.median(wl.input, 0, wl.views, states)):
+        np.testing.assert_array_equal(a.depth, b.depth)
+        np.testing.assert_array_equal(a.normal, b.normal)
