@@ -1835,34 +1835,49 @@ __global__ void __launch_bounds__(256) k_median(const __grid_constant__ PsRun P)
     return;
   }
   const float3 rp = pixel_ray(R, x, y);
-  float ds[25];
-  int qs[25];
+  // The depths of the 25 neighbours stay in registers (no depth: infinity), and the median is the one with (cnt - 1) / 2
+  // others before it in (depth, pixel) order, counted pair by pair.  An insertion sort in local memory, with the rays'
+  // divisions per neighbour, took 0.76 ms for 4 views of 640 × 480.
+  float rx[5], ry[5], ds[25];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    rx[k] = ((float)(x - 2 + k) - R.cx) / R.fx;  // pixel_ray's quotients
+    ry[k] = ((float)(y - 2 + k) - R.cy) / R.fy;
+  }
   int cnt = 0;
-  for (int qy = max(y - 2, 0); qy < min(y + 3, h); ++qy) {
-    for (int qx = max(x - 2, 0); qx < min(x + 3, w); ++qx) {
-      const float4 q = in[qy * w + qx];
-      if (!(q.w > 0.f)) continue;
-      const float3 n = make_float3(q.x, q.y, q.z);
-      const float den = dot3(n, rp);
-      if (!(den < -1e-6f)) continue;
-      const float d = q.w * dot3(n, pixel_ray(R, qx, qy)) / den;
-      if (!(d > 0.f) || !isfinite(d)) continue;
-      const int qi = qy * w + qx;
-      int k = cnt++;
-      while (k > 0 && (ds[k - 1] > d || (ds[k - 1] == d && qs[k - 1] > qi))) {
-        ds[k] = ds[k - 1];
-        qs[k] = qs[k - 1];
-        --k;
-      }
-      ds[k] = d;
-      qs[k] = qi;
-    }
+#pragma unroll
+  for (int k = 0; k < 25; ++k) {
+    const int qx = x - 2 + k % 5, qy = y - 2 + k / 5;
+    ds[k] = __int_as_float(0x7f800000);
+    if (qx < 0 || qy < 0 || qx >= w || qy >= h) continue;
+    const float4 q = in[qy * w + qx];
+    if (!(q.w > 0.f)) continue;
+    const float3 n = make_float3(q.x, q.y, q.z);
+    const float den = dot3(n, rp);
+    if (!(den < -1e-6f)) continue;
+    const float d = q.w * dot3(n, make_float3(rx[k % 5], ry[k / 5], 1.0f)) / den;
+    if (!(d > 0.f) || !isfinite(d)) continue;
+    ds[k] = d;
+    ++cnt;
   }
   float4 out = self;
   if (cnt > 0) {
     const int m = (cnt - 1) / 2;
-    const float4 q = in[qs[m]];
-    out = make_float4(q.x, q.y, q.z, ds[m]);
+    int at = 0;
+    float dm = 0.f;
+#pragma unroll
+    for (int k = 0; k < 25; ++k) {
+      int before = 0;
+#pragma unroll
+      for (int q = 0; q < 25; ++q)
+        if (q != k) before += q < k ? ds[q] <= ds[k] : ds[q] < ds[k];
+      if (before == m) {  // m < cnt: never one without depth
+        at = k;
+        dm = ds[k];
+      }
+    }
+    const float4 q = in[(y - 2 + at / 5) * w + x - 2 + at % 5];
+    out = make_float4(q.x, q.y, q.z, dm);
   }
   P.plane[it.off + y * w + x] = out;
 }
