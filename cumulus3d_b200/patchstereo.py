@@ -126,6 +126,31 @@ class DepthSnapshot:
     maps: List[Optional[np.ndarray]]
 
 
+def _out_arrays(sizes, channels: int = 1, dtype=np.float32, block_bytes: int = 1 << 24) -> List[np.ndarray]:
+    """One uninitialised flat array of w·h·channels values per (w, h), for calls that write all of them.  Fresh memory
+    costs a page fault per 4 KB; small views share blocks of up to `block_bytes`, which the allocator backs with large
+    pages (and a kept view keeps at most its block alive)."""
+    item = np.dtype(dtype).itemsize
+    out, i = [], 0
+    while i < len(sizes):
+        n, j = 0, i
+        while j < len(sizes) and (j == i or (n + sizes[j][0] * sizes[j][1] * channels) * item <= block_bytes):
+            n += sizes[j][0] * sizes[j][1] * channels
+            j += 1
+        block, o = np.empty(n, dtype), 0
+        for w, h in sizes[i:j]:
+            out.append(block[o:o + w * h * channels])
+            o += w * h * channels
+        i = j
+    return out
+
+
+def _out_states(sizes) -> List[ViewState]:
+    """Uninitialised states of the given sizes (see _out_arrays)."""
+    return [ViewState(w, h, a[:w * h].reshape(h, w), a[w * h:4 * w * h].reshape(h, w, 3), a[4 * w * h:].reshape(h, w))
+            for (w, h), a in zip(sizes, _out_arrays(sizes, 5))]
+
+
 class CInput:
     """Marshals a KernelInput into the C structs, keeping every referenced buffer alive."""
 
@@ -297,7 +322,7 @@ class PatchMatchSession:
                  snapshot: Optional[DepthSnapshot] = None) -> List[np.ndarray]:
         keep = []
         cs = c_states(states, keep)
-        outs = [np.empty((s.height, s.width), np.float32) for s in states]
+        outs = [a.reshape(s.height, s.width) for a, s in zip(_out_arrays([(s.width, s.height) for s in states]), states)]
         op = (FP * max(len(outs), 1))(*[_fptr(o) for o in outs])
         self._check(self.lib.ps_evaluate(self.h, level, _views(views), len(views), cs, int(geometric),
                                          c_snapshot(snapshot, keep), op))
@@ -315,7 +340,7 @@ class PatchMatchSession:
                  sigma_c: float) -> List[ViewState]:
         keep = []
         cl = c_states(low, keep)
-        outs = [ViewState.new(*self._size(v, level)) for v in views]
+        outs = _out_states([self._size(v, level) for v in views])
         co = c_states(outs, keep)
         self._check(self.lib.ps_upsample(self.h, level, _views(views), len(views), cl, sigma_s, sigma_c, co))
         return outs
@@ -324,11 +349,9 @@ class PatchMatchSession:
                       states: List[ViewState]) -> List[ViewState]:
         keep = []
         ci = c_states(states, keep)
-        outs = [ViewState.new(*self._size(v, level)) for v in views]
+        outs = _out_states([self._size(v, level) for v in views])
         co = c_states(outs, keep)
         self._check(self.lib.ps_median_filter(self.h, level, _views(views), len(views), ci, co))
-        for o, s in zip(outs, states):
-            o.cost[...] = s.cost
         return outs
 
     # ---- device-resident extension ----------------------------------------------------------------------------
@@ -338,7 +361,7 @@ class PatchMatchSession:
 
     def download(self, level: int, views: Sequence[int]) -> List[ViewState]:
         keep = []
-        outs = [ViewState.new(*self._size(v, level)) for v in views]
+        outs = _out_states([self._size(v, level) for v in views])
         self._check(self.lib.ps_state_download(self.h, level, _views(views), len(views), c_states(outs, keep)))
         return outs
 
@@ -380,7 +403,7 @@ class PatchMatchSession:
             return None
         keep = []
         lvl = self._snap_level_guess()
-        outs = [ViewState.new(*self._size(v, lvl)) for v in views]
+        outs = _out_states([self._size(v, lvl) for v in views])
         self._check(self.lib.ps_readout_resident(self.h, _views(views), len(views), c_states(outs, keep)))
         return outs
 
@@ -415,7 +438,7 @@ class PatchMatchSession:
 
     def readout_download(self, level: int, views: Sequence[int]) -> List[ViewState]:
         """The current readout planes (after post-processing) and costs, without recomputing the readout."""
-        out = [ViewState.new(*self._size(v, level)) for v in views]
+        out = _out_states([self._size(v, level) for v in views])
         keep = []
         self._check(self.lib.ps_readout_download(self.h, level, _views(views), len(views), c_states(out, keep)))
         return out
