@@ -2,10 +2,8 @@
 
 All variants of the half-step kernel produce the same bits, so the choice only affects speed:
 
-* lanes per pixel: one thread per pixel, or two lanes that split the window rows;
-* window-weight cache: on or off;
-* source sampling: loads from the bordered plane, or a texture gather;
-* row-pair f32x2 loops, staged source boxes (cp.async or TMA tensor loads), a persistent launch per run.
+* the default kernel (the words 0, 2, 3, 4, 6, 7, 8 and 10 all select it);
+* staged source boxes (cp.async or TMA tensor loads), a persistent launch per run.
 
 The tuner times each candidate on a prefix of the caller's own views and returns the fastest tuning word: a
 photometric run of two red-black iterations from random init brings the planes near convergence (the state most

@@ -3,7 +3,8 @@
 // It plays the role of the reference's CUDA session (crates/cuda/src/patchmatch.rs:285-1009): one session per
 // backend, one stream per session, every image of every level resident in HBM for the session's lifetime.  The
 // B200 design differs in these points:
-//   * images are uploaded once as normalised f32 planes with a zero border (no CUDA arrays / texture objects);
+//   * images are uploaded once, as normalised f32 planes with a zero border (reference tiles, TMA boxes) and as
+//     gather-capable texture arrays (source taps);
 //   * per-pixel state lives in per-level "slots" (plane float4, cost, best view, count, prior) that persist across
 //     calls, so the host-state calls (ps_run, ps_evaluate, …) are thin wrappers over resident ones and a caller that
 //     keeps everything on the device (ps_run_resident, ps_snapshot_capture, ps_filter_resident) never copies states;
@@ -692,6 +693,17 @@ void upload_planes(ps_session* s, const uint32_t* views, size_t a, size_t b, con
   sync(s);  // the staging buffer is reused by the next call
 }
 
+// Writes every page of an output array once (its own byte back), so that fresh memory takes its page faults here.
+void touch_pages(void* p, size_t bytes) {
+  char* const b = (char*)p;
+  const long long n = (long long)(bytes / 4096);
+#pragma omp parallel for schedule(static) if (n > 64)
+  for (long long i = 0; i < n; ++i) {
+    volatile char* const q = b + i * 4096;
+    *q = *q;
+  }
+}
+
 // Downloads planes (from `src` or the slot planes) and/or costs into host states.
 void download_states(ps_session* s, const uint32_t* views, size_t a, size_t b, ps_view_state* states, int level,
                      bool planes, bool costs, const float4* src = nullptr) {
@@ -721,6 +733,16 @@ void download_states(ps_session* s, const uint32_t* views, size_t a, size_t b, p
               "download cost");
     cuda_ok(cudaEventRecord(s->xfer[i - a], s->st), "cudaEventRecord");
     o += n;
+  }
+  // the states' pages are made present while the stream still works (a schedule before the download, the copies): their
+  // faults take as long as the copies, 8.7 against 15.5 ms for 5 views of 1920 × 1080 on pages that are there
+  for (size_t i = a; i < b; ++i) {
+    const size_t n = (size_t)states[i].width * states[i].height;
+    if (planes) {
+      touch_pages(states[i].normal, 3 * n * sizeof(float));
+      touch_pages(states[i].depth, n * sizeof(float));
+    }
+    if (costs) touch_pages(states[i].cost, n * sizeof(float));
   }
   // each view is unpacked as soon as its own copies are done, while the later views' copies run
   for (size_t i = a; i < b; ++i) {

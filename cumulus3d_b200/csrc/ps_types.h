@@ -1,7 +1,7 @@
 // Device-side descriptor tables of the PatchStereo engine (plain structs shared by the kernels and the host
 // runtime).  They play the role of the reference's LevelDesc / PairRec / LevelPair / ViewDesc / BatchItem / KParams
 // (crates/cuda/src/kernels/patchmatch.cu:52-109), laid out for this engine: images are normalised f32 planes with a
-// zero border instead of texture objects, and the batch table travels inside the kernel parameters.
+// zero border beside their texture objects, and the batch table travels inside the kernel parameters.
 #pragma once
 #include <stdint.h>
 
