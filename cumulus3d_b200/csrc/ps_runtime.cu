@@ -2231,8 +2231,16 @@ int ps_postprocess_resident(ps_session* s, uint32_t level, const uint32_t* views
     if (!s->pcount) s->pcount = dalloc<unsigned long long>(s, 3);
     cuda_ok(cudaMemsetAsync(s->pcount, 0, 2 * sizeof(unsigned long long), s->st), "memset");
     const size_t T = (size_t)std::max<long long>(sl.total, 1);
+    // A view named more than once is cleaned once: twice in one launch its pixels would count double, and its runs of cost
+    // keys would not fit A.hi, which has one word per pixel of the distinct views.
+    std::vector<uint32_t> once;
+    std::vector<char> named(s->nv, 0);
+    for (size_t i = 0; i < n; ++i) {
+      if (!named[views[i]]) once.push_back(views[i]);
+      named[views[i]] = 1;
+    }
     if (p->remove_speckles)
-    for (auto [a, b] : batches(s, views, n, (int)level)) {
+    for (auto [a, b] : batches(s, once.data(), once.size(), (int)level)) {
       ps_post::SpkArgs A;
       memset(&A, 0, sizeof A);
       A.plane = sl.aux;
@@ -2246,7 +2254,7 @@ int ps_postprocess_resident(ps_session* s, uint32_t level, const uint32_t* views
       A.nkeys = reinterpret_cast<unsigned*>(s->pcount + 2);
       A.rel = p->speckle_rel_depth;
       A.keep = p->speckle_keep_cost;
-      const int tiles = spk_items(s, A, views, a, b, (int)level, p->speckle_min_area_frac);
+      const int tiles = spk_items(s, A, once.data(), a, b, (int)level, p->speckle_min_area_frac);
       bool any = false;
       for (int i = 0; i < A.nitems; ++i) any = any || A.items[i].min_area > 1;
       if (!any) continue;  // the reference returns early when the minimum area is <= 1

@@ -427,7 +427,8 @@ int ps_proposal_download(ps_session* s, uint32_t level, const uint32_t* views, s
  * PostParams (crates/dense/src/postproc.rs:41-74), applied to the readout planes of `level` in place, in the
  * reference's order (crates/dense/src/densify.rs:455-461):
  *  - remove_speckles (postproc.rs:77-129): 4-connected components (|d_j - d_i| <= rel·min(d_i, d_j)) smaller than
- *    ceil(w·h·min_area_frac) whose lower median cost exceeds keep_cost are erased;
+ *    ceil(w·h·min_area_frac) whose lower median cost exceeds keep_cost are erased (once per view, also when `views`
+ *    names it more than once);
  *  - fill_holes (postproc.rs:139-201, off by default): every invalid pixel whose run cost is at most fill_max_cost
  *    walks the 8 directions up to round(diag·fill_max_frac) steps over the 8-bit gray image, stopping where the gray
  *    value jumps by more than fill_edge_step·255, and takes the plane of the valid pixel it meets with the smallest

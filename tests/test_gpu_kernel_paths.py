@@ -91,6 +91,29 @@ def test_speckles_at_tile_edges(w, h, frac):
     assert removed == n
 
 
+@pytest.mark.parametrize("repeat,max_batch", [([0, 0], 64), ([1, 0, 1, 1, 2, 0], 64), ([0, 1, 0, 2, 2], 2)])
+def test_speckles_of_views_named_more_than_once(repeat, max_batch):
+    """Within one launch and across launches: each view is cleaned once, and its erased pixels count once."""
+    wl = scenes.workload_small(40, 24, views=3, window_radius=3, seed=11)
+    post = fusion.default_post()
+    post.speckle_min_area_frac = 0.2
+    be = PatchMatchBackend(0, max_batch=max_batch)
+    with be.begin(wl.input) as s:
+        s.schedule_resident(wl.views, 1, 0, 0)
+        before = s.readout_resident(wl.views)
+        removed = s.postprocess_resident(0, repeat, post)
+        after = s.readout_download(0, wl.views)
+    be.close()
+    n = 0
+    for v, (b, a) in enumerate(zip(before, after)):
+        d, nn = b.depth.copy(), b.normal.copy()
+        if v in repeat:
+            n += oracle.remove_speckles(d, nn, b.cost, post)
+        np.testing.assert_array_equal(a.depth, d)
+        np.testing.assert_array_equal(a.normal, nn)
+    assert removed == n and n > 0
+
+
 @pytest.mark.parametrize("w,h", [(1, 1), (2, 5), (33, 9)])
 def test_median_at_edges_and_ties(w, h):
     wl = scenes.workload_small(w, h, views=2, window_radius=1, seed=3, sources=1)
