@@ -2045,6 +2045,8 @@ static bool compiled_window(int wr, int ws) {
 static bool half_staged(unsigned tuning, int wr, int ws) {
   return (tuning & 0x10u) && !(tuning & 0x1u) && compiled_window(wr, ws);
 }
+// Whether the half steps of this tuning word and window read the costs that a run keeps (PsRun::kept).
+bool half_keeps(unsigned tuning, int wr, int ws) { return !half_staged(tuning, wr, ws); }
 
 // Whether the persistent kernel runs a run's half steps for this tuning word and window: PS_TUNE_PERSISTENT with
 // PS_TUNE_ROW_PAIRS at a compiled window.

@@ -34,6 +34,7 @@
   namespace NS {                                                                                           \
   cudaError_t launch_half(const PsRun& P, unsigned tuning, cudaStream_t st);                               \
   bool half_run_ok(unsigned tuning, int wr, int ws);                                                       \
+  bool half_keeps(unsigned tuning, int wr, int ws);                                                        \
   cudaError_t launch_half_run(const PsRun& P, unsigned tuning, cudaStream_t st);                           \
   cudaError_t launch_eval(const PsRun& P, cudaStream_t st);                                                \
   cudaError_t launch_filter(const PsRun& P, cudaStream_t st);                                              \
@@ -67,19 +68,23 @@ struct Launchers {
   cudaError_t (*restore)(const PsRun&, const float4*, const float*, float, cudaStream_t);
   bool (*half_run_ok)(unsigned, int, int);
   cudaError_t (*half_run)(const PsRun&, unsigned, cudaStream_t);
+  bool (*half_keeps)(unsigned, int, int);
 };
 const Launchers kParity = {ps_parity::launch_half,     ps_parity::launch_eval,   ps_parity::launch_filter,
                            ps_parity::launch_upsample, ps_parity::launch_median, ps_parity::launch_snapshot,
                            ps_parity::launch_readout,  ps_parity::launch_sweep,
-                           ps_parity::launch_restore, ps_parity::half_run_ok, ps_parity::launch_half_run};
+                           ps_parity::launch_restore, ps_parity::half_run_ok, ps_parity::launch_half_run,
+                           ps_parity::half_keeps};
 const Launchers kFast = {ps_fast::launch_half,     ps_fast::launch_eval,   ps_fast::launch_filter,
                          ps_fast::launch_upsample, ps_fast::launch_median, ps_fast::launch_snapshot,
                          ps_fast::launch_readout,  ps_fast::launch_sweep,
-                         ps_fast::launch_restore, ps_fast::half_run_ok, ps_fast::launch_half_run};
+                         ps_fast::launch_restore, ps_fast::half_run_ok, ps_fast::launch_half_run,
+                         ps_fast::half_keeps};
 const Launchers kChecked = {ps_checked::launch_half,     ps_checked::launch_eval,   ps_checked::launch_filter,
                             ps_checked::launch_upsample, ps_checked::launch_median, ps_checked::launch_snapshot,
                             ps_checked::launch_readout,  ps_checked::launch_sweep,
-                            ps_checked::launch_restore, ps_checked::half_run_ok, ps_checked::launch_half_run};
+                            ps_checked::launch_restore, ps_checked::half_run_ok, ps_checked::launch_half_run,
+                            ps_checked::half_keeps};
 
 struct PsError {
   int code;
@@ -218,6 +223,7 @@ struct ps_session {
   double* pairs64 = nullptr;
   int* has64 = nullptr;
   std::vector<Slot> slots;
+  bool no_kept = false;  // device memory ran short: runs of this session keep no costs (PsRun::kept)
   // snapshot
   float* snap = nullptr;
   size_t snap_cap = 0;
@@ -350,16 +356,30 @@ void check_fault(ps_session* s) {
                       "); the access was skipped");
 }
 
+bool reclaim(ps_session* s);  // below: gives back device memory that only saves work
+
 // Session device memory: from the backend's pool in the session stream's order (plain cudaMalloc when the device
-// offers no pool).  Every use of a buffer is on the session stream.
+// offers no pool).  Every use of a buffer is on the session stream.  `optional`: the caller does without when it fails.
 template <typename T>
-T* dalloc(ps_session* s, size_t n) {
-  maybe_inject(s, PS_INJECT_DEVICE_ALLOC, "device allocation");
-  void* p = nullptr;
+T* dalloc(ps_session* s, size_t n, bool optional = false) {
   const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
-  if (s->be && s->be->pool) cuda_ok(cudaMallocFromPoolAsync(&p, bytes, s->be->pool, s->st), "cudaMallocFromPoolAsync");
-  else cuda_ok(cudaMalloc(&p, bytes), "cudaMalloc");
-  return (T*)p;
+  try {
+    maybe_inject(s, PS_INJECT_DEVICE_ALLOC, "device allocation");
+  } catch (const PsError&) {
+    if (optional || !reclaim(s)) throw;
+  }
+  void* p = nullptr;
+  for (bool again = !optional;; again = false) {
+    const bool pool = s->be && s->be->pool;
+    const cudaError_t e = pool ? cudaMallocFromPoolAsync(&p, bytes, s->be->pool, s->st) : cudaMalloc(&p, bytes);
+    if (e == cudaErrorMemoryAllocation && again && !s->capturing) {
+      cudaGetLastError();
+      reclaim(s);
+      continue;
+    }
+    cuda_ok(e, pool ? "cudaMallocFromPoolAsync" : "cudaMalloc");
+    return (T*)p;
+  }
 }
 void dfree(ps_session* s, void* p) {
   if (!p) return;
@@ -400,17 +420,6 @@ Slot& slot(ps_session* s, int level) {
     sl.aux = dalloc<float4>(s, tot);
     sl.prior = dalloc<float4>(s, tot);
     sl.cost = dalloc<float>(s, tot);
-    {  // the kept costs only save work: without memory for them the run does without
-      const int most = s->nsrc.empty() ? 0 : *std::max_element(s->nsrc.begin(), s->nsrc.end());
-      void* k = nullptr;
-      sl.keep = std::min(most, PS_KEEP);
-      const size_t bytes = (size_t)std::max<long long>(tot, 1) * sl.keep * sizeof(float);
-      if (sl.keep > 0 && s->be && s->be->pool && cudaMallocFromPoolAsync(&k, bytes, s->be->pool, s->st) != cudaSuccess) {
-        cudaGetLastError();
-        k = nullptr;
-      }
-      sl.kept = (float*)k;
-    }
     sl.bview = dalloc<unsigned char>(s, tot);
     sl.count = dalloc<unsigned char>(s, tot);
     cuda_ok(cudaMemsetAsync(sl.plane, 0, std::max<long long>(tot, 1) * sizeof(float4), s->st), "memset");
@@ -419,6 +428,23 @@ Slot& slot(ps_session* s, int level) {
     sl.ready = true;
   }
   return sl;
+}
+
+// The buffer in which the runs of a level keep costs (PsRun::kept): made by the first run whose half steps read it, outside
+// captures, after what the call cannot do without.  It only saves work, so without memory for it the session's runs do
+// without, and reclaim() gives it back when another allocation fails.
+void keep_costs(ps_session* s, int level) {
+  Slot& sl = slot(s, level);
+  if (sl.kept || s->no_kept || !s->be || !s->be->pool) return;
+  if (!s->L->half_keeps(s->tuning, s->pm.window_radius, s->pm.window_step)) return;
+  sl.keep = std::min(s->nsrc.empty() ? 0 : *std::max_element(s->nsrc.begin(), s->nsrc.end()), PS_KEEP);
+  if (sl.keep < 1) return;
+  try {
+    sl.kept = dalloc<float>(s, (size_t)std::max<long long>(sl.total, 1) * sl.keep, true);
+  } catch (const PsError& e) {
+    if (e.code != PS_ENOMEM) throw;
+    s->no_kept = true;
+  }
 }
 
 // Splits a view list into launches of at most max_batch views and batch_pixels pixels (cf. Session::batches,
@@ -629,6 +655,28 @@ void drop_graphs(ps_session* s) {
     }
   }
   s->graphs.clear();
+}
+
+// An allocation failed: gives back the kept costs (the captured graphs that hold their address with them) and the pool's
+// unused memory.  Returns whether a buffer was given back.
+bool reclaim(ps_session* s) {
+  if (s->capturing) return false;
+  if (s->st) cudaStreamSynchronize(s->st);  // no graph runs any more
+  bool freed = false;
+  for (Slot& sl : s->slots) {
+    if (!sl.kept) continue;
+    drop_graphs(s);
+    dfree(s, sl.kept);
+    sl.kept = nullptr;
+    s->no_kept = true;
+    freed = true;
+  }
+  if (s->be && s->be->pool && s->st) {
+    cudaStreamSynchronize(s->st);  // what was freed in stream order is unused now
+    cudaMemPoolTrimTo(s->be->pool, 0);
+    cudaGetLastError();
+  }
+  return freed;
 }
 
 // Grows the snapshot buffer to `total` floats (captured graphs are dropped first).
@@ -1323,6 +1371,7 @@ int ps_run_resident(ps_session* s, const uint32_t* views, size_t n, const ps_run
     check_views(s, views, n);
     Slot& sl = slot(s, (int)p->level);
     if (p->geometric) require_snapshot_level(s, (int)p->level);
+    keep_costs(s, (int)p->level);
     for (auto [a, b] : batches(s, views, n, (int)p->level)) {
       bool up = p->use_prior != 0;
       for (size_t i = a; i < b; ++i) up = up && sl.prior_valid[views[i]];
@@ -1449,6 +1498,7 @@ int ps_run(ps_session* s, const uint32_t* views, size_t n, ps_view_state* states
     if (p->geometric && s->snap_level != (int)p->level) fail(PS_EINVAL, "snapshot level differs from the run level");
     const int level = (int)p->level;
     Slot& sl = slot(s, level);
+    keep_costs(s, level);
     for (auto [a, b] : batches(s, views, n, level)) {
       for (size_t i = a; i < b; ++i) check_state(s, (int)views[i], level, states[i]);
       size_t px = 0;
@@ -1914,7 +1964,10 @@ int ps_schedule_resident(ps_session* s, const uint32_t* views, size_t n, const p
     for (size_t i = 0; i < n; ++i) key += std::to_string(views[i]) + ",";
     graph_run(
         s, key, sch->use_graph != 0,
-        [&](ps_session::GraphEntry& ge) { ge.offsets = view_offsets(s, level, views, n); },
+        [&](ps_session::GraphEntry& ge) {
+          ge.offsets = view_offsets(s, level, views, n);
+          keep_costs(s, level);
+        },
         [&](ps_session::GraphEntry& ge) { enqueue_schedule(s, views, n, sch, ge.offsets); });
     s->snap_valid = true;
     s->snap_level = level;
@@ -1961,6 +2014,7 @@ int ps_schedule_multiscale(ps_session* s, const uint32_t* views, size_t n, const
         s, key, m->use_graph != 0,
         [&](ps_session::GraphEntry& ge) {
           for (int l = 0; l < s->nl; ++l) ge.level_offsets.push_back(view_offsets(s, l, views, n));
+          for (int l = 0; l < s->nl; ++l) keep_costs(s, l);
         },
         [&](ps_session::GraphEntry& ge) { enqueue_multiscale(s, views, n, m, ge.level_offsets); });
     s->snap_valid = true;
@@ -2066,7 +2120,11 @@ int ps_propose(ps_session* s, ps_net* net, uint32_t level, const uint32_t* views
         cuda_ok(cudaEventRecord(pd.a, s->st), "cudaEventRecord");
       }
       std::string err;
-      const int rc = ps_cnn::forward_on_stream(net, s->netin, 1, hp, wp, s->netout, s->st, &err);
+      int rc = ps_cnn::forward_on_stream(net, s->netin, 1, hp, wp, s->netout, s->st, &err);
+      if (rc == PS_ENOMEM) {  // the network's workspace is outside the pool
+        reclaim(s);
+        rc = ps_cnn::forward_on_stream(net, s->netin, 1, hp, wp, s->netout, s->st, &err);
+      }
       if (rc != PS_OK) {
         if (s->profiling) {
           cudaEventDestroy(pd.a);

@@ -4,6 +4,8 @@ mapping (crates/cuda/src/patchmatch.rs:234-236, :258, :292-294, :641) and a back
 * a second session on a busy backend: PS_EBUSY (the reference's backend holds a mutex for the session's life);
 * an injected device-allocation failure: PS_ENOMEM from ps_begin; an injected upload failure: PS_ECUDA from ps_begin
   and from ps_run; each time the next session or call runs normally and equals the CPU oracle bit for bit;
+* memory for the costs that runs keep fails, or is wanted back by another allocation: the calls run without it, to the
+  same bits;
 * malformed states (NaN, infinite and negative depths, NaN normals) run to completion with the oracle's bits;
 * a snapshot map of the wrong size is left out, as the reference leaves it out, and a snapshot of another level is
   rejected with PS_EINVAL.
@@ -97,6 +99,71 @@ def test_injected_upload_failures():
     want = _oracle_run(wl, p)
     oracle.run(wl.input, wl.views, want, cont)
     _same(got, want, "after an upload failure")
+
+
+SLOT_ALLOCS = 6  # device allocations of a level's state, before the one for the costs that its runs keep
+
+
+@pytest.mark.parametrize("tuning", [0, 42])
+def test_run_without_memory_for_kept_costs(tuning):
+    """The allocation for the kept costs fails (the failure is spent there: the geometric run allocates its snapshot):
+    runs without them, the oracle's bits."""
+    wl = _wl()
+    p, g = RunParams(0, False, True, 2, 1), RunParams(0, True, False, 2, 2)
+    be = PatchMatchBackend(0, tuning=tuning)
+    got, want = _states(wl), _oracle_run(wl, p)
+    with be.begin(wl.input) as s:
+        be.inject_failure(_lib.PS_INJECT_DEVICE_ALLOC, SLOT_ALLOCS)
+        s.run(wl.views, got, p)
+        _same(got, want, "photometric run")
+        snap = DepthSnapshot(1, 0, [x.depth.copy() for x in got])
+        s.run(wl.views, got, g, snap)
+    be.close()
+    _same(got, _oracle_run(wl, g, want, snap), "geometric run")
+
+
+def test_kept_costs_are_given_back_to_other_allocations():
+    """The snapshot's allocation fails while a run's kept costs hold memory, then the speckle buffer's while a captured
+    schedule holds their address: both calls succeed, and what runs afterwards has the same bits."""
+    wl = _wl()
+    p, g = RunParams(0, False, True, 2, 1), RunParams(0, True, False, 2, 2)
+    be = PatchMatchBackend(0)
+    got, want = _states(wl), _oracle_run(wl, p)
+    with be.begin(wl.input) as s:
+        s.run(wl.views, got, p)
+        snap = DepthSnapshot(1, 0, [x.depth.copy() for x in got])
+        be.inject_failure(_lib.PS_INJECT_DEVICE_ALLOC, 0)
+        s.run(wl.views, got, g, snap)
+    _same(got, _oracle_run(wl, g, want, snap), "geometric run")
+    maps = []
+    with be.begin(wl.input) as s:
+        for fail in (True, False):
+            s.schedule_resident(wl.views, 2, 1, 1)
+            maps.append(s.readout_resident(wl.views))
+            if fail:
+                be.inject_failure(_lib.PS_INJECT_DEVICE_ALLOC, 0)
+            s.postprocess_resident(0, wl.views)
+    be.close()
+    _same(maps[1], maps[0], "schedule")
+
+
+@pytest.mark.parametrize("tuning,call", [(16, "run"), (0, "evaluate")])
+def test_no_kept_costs_where_nothing_reads_them(tuning, call):
+    """Staged half steps and evaluations allocate none: the failure behind the level's own allocations is still armed
+    for the snapshot."""
+    wl = _wl()
+    st = _states(wl)
+    be = PatchMatchBackend(0, tuning=tuning)
+    with be.begin(wl.input) as s:
+        be.inject_failure(_lib.PS_INJECT_DEVICE_ALLOC, SLOT_ALLOCS)
+        if call == "run":
+            s.run(wl.views, st, RunParams(0, False, True, 1, 1))
+        else:
+            s.evaluate(0, wl.views, st)
+        with pytest.raises(PsError) as e:
+            s.filter(wl.views, st, DepthSnapshot(1, 0, [x.depth.copy() for x in st]))
+        assert e.value.code == _lib.PS_ENOMEM
+    be.close()
 
 
 def test_malformed_states_run_like_the_oracle():
