@@ -358,28 +358,39 @@ void check_fault(ps_session* s) {
 
 bool reclaim(ps_session* s);  // below: gives back device memory that only saves work
 
+// One device allocation; unless it is optional, a failed one is tried once more after reclaim().
+template <typename F>
+void alloc_retried(ps_session* s, bool optional, const char* what, F&& alloc) {
+  try {
+    maybe_inject(s, PS_INJECT_DEVICE_ALLOC, what);
+  } catch (const PsError&) {
+    if (optional || !reclaim(s)) throw;
+  }
+  cudaError_t e = alloc();
+  if (e == cudaErrorMemoryAllocation && !optional && !s->capturing) {
+    cudaGetLastError();
+    reclaim(s);
+    e = alloc();
+  }
+  cuda_ok(e, what);
+}
+
 // Session device memory: from the backend's pool in the session stream's order (plain cudaMalloc when the device
 // offers no pool).  Every use of a buffer is on the session stream.  `optional`: the caller does without when it fails.
 template <typename T>
 T* dalloc(ps_session* s, size_t n, bool optional = false) {
   const size_t bytes = std::max<size_t>(n, 1) * sizeof(T);
-  try {
-    maybe_inject(s, PS_INJECT_DEVICE_ALLOC, "device allocation");
-  } catch (const PsError&) {
-    if (optional || !reclaim(s)) throw;
-  }
   void* p = nullptr;
-  for (bool again = !optional;; again = false) {
-    const bool pool = s->be && s->be->pool;
-    const cudaError_t e = pool ? cudaMallocFromPoolAsync(&p, bytes, s->be->pool, s->st) : cudaMalloc(&p, bytes);
-    if (e == cudaErrorMemoryAllocation && again && !s->capturing) {
-      cudaGetLastError();
-      reclaim(s);
-      continue;
-    }
-    cuda_ok(e, pool ? "cudaMallocFromPoolAsync" : "cudaMalloc");
-    return (T*)p;
-  }
+  alloc_retried(s, optional, "device allocation", [&] {
+    return s->be && s->be->pool ? cudaMallocFromPoolAsync(&p, bytes, s->be->pool, s->st) : cudaMalloc(&p, bytes);
+  });
+  return (T*)p;
+}
+// A gather-capable array (outside the pool).
+cudaArray_t array_alloc(ps_session* s, const cudaChannelFormatDesc& fmt, int w, int h) {
+  cudaArray_t a = nullptr;
+  alloc_retried(s, false, "texture array", [&] { return cudaMallocArray(&a, &fmt, w, h, cudaArrayTextureGather); });
+  return a;
 }
 void dfree(ps_session* s, void* p) {
   if (!p) return;
@@ -657,8 +668,9 @@ void drop_graphs(ps_session* s) {
   s->graphs.clear();
 }
 
-// An allocation failed: gives back the kept costs (the captured graphs that hold their address with them) and the pool's
-// unused memory.  Returns whether a buffer was given back.
+// An allocation failed: gives back the kept costs (the captured graphs that hold their address with them), the texture
+// arrays that wait for a session that may reuse them, and the pool's unused memory.  Returns whether a buffer or an array
+// was given back.
 bool reclaim(ps_session* s) {
   if (s->capturing) return false;
   if (s->st) cudaStreamSynchronize(s->st);  // no graph runs any more
@@ -669,6 +681,11 @@ bool reclaim(ps_session* s) {
     dfree(s, sl.kept);
     sl.kept = nullptr;
     s->no_kept = true;
+    freed = true;
+  }
+  if (s->be && !s->be->arrays.empty()) {
+    for (auto& c : s->be->arrays) cudaFreeArray(c.a);
+    s->be->arrays.clear();
     freed = true;
   }
   if (s->be && s->be->pool && s->st) {
@@ -1162,8 +1179,7 @@ int ps_begin(ps_backend* be, const ps_kernel_input* in, ps_session** out) {
               cache.erase(cache.begin() + (long)k);
               break;
             }
-          if (!arr)
-            cuda_ok(cudaMallocArray(&arr, u8 ? &cd8 : &cdf, L.w, L.h, cudaArrayTextureGather), "cudaMallocArray");
+          if (!arr) arr = array_alloc(s, u8 ? cd8 : cdf, L.w, L.h);
           s->arrays.push_back(arr);
           s->array_keys.push_back({arr, L.w, L.h, u8});
           if (u8)

@@ -207,7 +207,8 @@ typedef struct ps_session ps_session;
 
 /* ---- host-side failure injection (no counterpart in the reference; for tests of the error paths) ----------
  * Arms one failure on the backend: after `after` more operations of `kind` succeed, the next one fails as a device
- * would (PS_INJECT_DEVICE_ALLOC: a device allocation, reported as PS_ENOMEM; PS_INJECT_UPLOAD: a host-to-device copy
+ * would (PS_INJECT_DEVICE_ALLOC: a device allocation, reported as PS_ENOMEM unless memory that only saves work could be
+ * given back for it; PS_INJECT_UPLOAD: a host-to-device copy
  * of images, states or snapshots, reported as PS_ECUDA), then the injection disarms itself.  PS_INJECT_NONE disarms.
  * Nothing reaches the GPU: the failing operation is refused on the host before it is issued. */
 #define PS_INJECT_NONE 0u

@@ -2,8 +2,8 @@
 mapping (crates/cuda/src/patchmatch.rs:234-236, :258, :292-294, :641) and a backend that stays usable afterwards.
 
 * a second session on a busy backend: PS_EBUSY (the reference's backend holds a mutex for the session's life);
-* an injected device-allocation failure: PS_ENOMEM from ps_begin; an injected upload failure: PS_ECUDA from ps_begin
-  and from ps_run; each time the next session or call runs normally and equals the CPU oracle bit for bit;
+* an injected device-allocation failure: PS_ENOMEM from ps_begin, unless the backend holds texture arrays to give back;
+  an injected upload failure: PS_ECUDA from ps_begin and from ps_run; each time the next session or call runs normally and equals the CPU oracle bit for bit;
 * memory for the costs that runs keep fails, or is wanted back by another allocation: the calls run without it, to the
   same bits;
 * malformed states (NaN, infinite and negative depths, NaN normals) run to completion with the oracle's bits;
@@ -73,6 +73,23 @@ def test_injected_device_allocation_failure(after):
         s.run(wl.views, got, p)
     be.close()
     _same(got, _oracle_run(wl, p), f"after an allocation failure ({after})")
+
+
+@pytest.mark.parametrize("after", [1, 3])
+def test_waiting_texture_arrays_are_given_back(after):
+    """The image planes' allocation (1) or the first texture array's (3) fails in ps_begin while the backend holds the
+    arrays of an earlier session of other sizes: they are freed and the session begins."""
+    be = PatchMatchBackend(0)
+    be.begin(scenes.workload_small(120, 40, views=2, window_radius=3, seed=3).input).close()
+    wl = _wl()
+    p = RunParams(0, False, True, 2, 1)
+    got = _states(wl)
+    be.inject_failure(_lib.PS_INJECT_DEVICE_ALLOC, after)
+    with be.begin(wl.input) as s:
+        s.run(wl.views, got, p)
+    be.inject_failure(_lib.PS_INJECT_NONE)
+    be.close()
+    _same(got, _oracle_run(wl, p), f"after {after}")
 
 
 def test_injected_upload_failures():
