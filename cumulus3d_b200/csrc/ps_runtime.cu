@@ -758,14 +758,17 @@ void upload_planes(ps_session* s, const uint32_t* views, size_t a, size_t b, con
   sync(s);  // the staging buffer is reused by the next call
 }
 
-// Writes every page of an output array once (its own byte back), so that fresh memory takes its page faults here.
-void touch_pages(void* p, size_t bytes) {
-  char* const b = (char*)p;
-  const long long n = (long long)(bytes / 4096);
+// Writes the pages of an output array (their own bytes back) while the stream has not reached `reached`, so that fresh
+// memory takes its page faults meanwhile.  One locked write per page: a read first would map the zero page, and the large
+// pages of the allocator would be split.
+void touch_pages(void* p, size_t bytes, cudaEvent_t reached) {
+  constexpr size_t kChunk = size_t(4) << 20;
+  for (size_t at = 0; at < bytes; at += kChunk) {
+    if (cudaEventQuery(reached) != cudaErrorNotReady) return;
+    char* const b = (char*)p + at;
+    const long long n = (long long)((std::min(kChunk, bytes - at) + 4095) / 4096);
 #pragma omp parallel for schedule(static) if (n > 64)
-  for (long long i = 0; i < n; ++i) {
-    volatile char* const q = b + i * 4096;
-    *q = *q;
+    for (long long i = 0; i < n; ++i) __atomic_fetch_or(b + i * 4096, 0, __ATOMIC_RELAXED);
   }
 }
 
@@ -784,7 +787,9 @@ void download_states(ps_session* s, const uint32_t* views, size_t a, size_t b, p
   }
   size_t o = 0;
   std::vector<size_t> so;
-  xfer_events(s, b - a);
+  xfer_events(s, b - a + 1);
+  const cudaEvent_t reached = s->xfer[b - a];  // what the stream had to do before the copies is done
+  cuda_ok(cudaEventRecord(reached, s->st), "cudaEventRecord");
   for (size_t i = a; i < b; ++i) {
     const int v = (int)views[i];
     const size_t n = (size_t)s->W(v, level) * s->H(v, level);
@@ -799,17 +804,19 @@ void download_states(ps_session* s, const uint32_t* views, size_t a, size_t b, p
     cuda_ok(cudaEventRecord(s->xfer[i - a], s->st), "cudaEventRecord");
     o += n;
   }
-  // the states' pages are made present while the stream still works (a schedule before the download, the copies): their
-  // faults take as long as the copies, 8.7 against 15.5 ms for 5 views of 1920 × 1080 on pages that are there.  Only from
-  // 2^22 pixels on: with less, nothing long runs meanwhile (4 calls on 4 views of 640 × 480 took 15.3 ms so, 8.6 to 9.6 without).
-  for (size_t i = a; i < b && total >= (size_t(1) << 22); ++i) {
+  // The states' pages are made present while the stream still works on what came before the copies, not beyond (ms, never
+  // / always with a read first / this rule; after a run of two iterations and with nothing before the copies: 4 views of
+  // 640 × 480 14.1 / 12.5 / 12.5 and 2.4 / 8.5 / 2.2, 3 of 1280 × 720 30.1 / 28.3 / 28.5 and 3.9 / 11.9 / 3.5, 5 of
+  // 1920 × 1080 117.5 / 111.5 / 111.8 and 14.7 / 26.0 / 14.6, 12 of 1920 × 1080 282 / 269 / 269 and 36 / 62 / 34).
+  for (size_t i = a; i < b; ++i) {
     const size_t n = (size_t)states[i].width * states[i].height;
     if (planes) {
-      touch_pages(states[i].normal, 3 * n * sizeof(float));
-      touch_pages(states[i].depth, n * sizeof(float));
+      touch_pages(states[i].normal, 3 * n * sizeof(float), reached);
+      touch_pages(states[i].depth, n * sizeof(float), reached);
     }
-    if (costs) touch_pages(states[i].cost, n * sizeof(float));
+    if (costs) touch_pages(states[i].cost, n * sizeof(float), reached);
   }
+  cudaGetLastError();  // "not ready" is no error
   // each view is unpacked as soon as its own copies are done, while the later views' copies run
   for (size_t i = a; i < b; ++i) {
     cuda_ok(cudaEventSynchronize(s->xfer[i - a]), "cudaEventSynchronize");

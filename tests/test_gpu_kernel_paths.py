@@ -1,10 +1,11 @@
 """Device paths at the sizes where they can go wrong, against the CPU oracle bit for bit: windows without a kernel of their
-own, the costs a run keeps (more sources than it keeps, planes without depth), the speckle tiles' edges, the median's."""
+own, the costs a run keeps (more sources than it keeps, planes without depth), the speckle tiles' edges, the median's,
+downloads beside running work."""
 import numpy as np
 import pytest
 
 from cumulus3d_b200 import fusion, scenes
-from cumulus3d_b200.patchstereo import DepthSnapshot, PatchMatchBackend, RunParams, ViewState
+from cumulus3d_b200.patchstereo import DepthSnapshot, PatchMatchBackend, RunParams, ViewState, _views, c_states
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -131,3 +132,31 @@ def test_median_at_edges_and_ties(w, h):
     for a, b in zip(got, oracle.median(wl.input, 0, wl.views, states)):
         np.testing.assert_array_equal(a.depth, b.depth)
         np.testing.assert_array_equal(a.normal, b.normal)
+
+
+@pytest.mark.parametrize("sizes", [[(1, 1)], [(31, 33), (640, 480)], [(801, 603), (67, 13), (801, 603), (1300, 900)]])
+def test_downloads_with_and_without_pending_work(sizes):
+    """States downloaded while their run is still in flight (pages made present meanwhile, in chunks of 4 MB) hold what an
+    idle download holds; arrays of several views in one block, of one view alone, and arrays that had other values."""
+    cams = [scenes.formation(w, h, 1, prefix=f"d{i}")[0] for i, (w, h) in enumerate(sizes)]
+    cams.append(scenes.formation(64, 48, 1, prefix="src")[1])
+    rng = np.random.default_rng(9)
+    img = [rng.random((c.height, c.width), np.float32) for c in cams]
+    n = len(sizes)
+    inp = scenes.kernel_input(cams, img, [[n]] * n + [[0]], (25.0, 60.0), window_radius=3)
+    views = list(range(n))
+    be = PatchMatchBackend(0)
+    with be.begin(inp) as s:
+        for p in (RunParams(0, False, True, 3, 1), RunParams(0, False, False, 2, 2)):
+            s.run_resident(views, p)
+            pending = s.download(0, views)
+            idle = s.download(0, views)
+            host = [ViewState.new(w, h) for w, h in sizes]
+            for st in host:
+                st.depth[...], st.normal[...], st.cost[...] = 7.0, 8.0, 9.0
+            s._check(s.lib.ps_state_download(s.h, 0, _views(views), n, c_states(host, [])))
+            for a, b, c in zip(pending, idle, host):
+                _same(a, b, "pending, idle")
+                _same(a, c, "pending, filled")
+                assert (a.depth > 0).all()
+    be.close()
