@@ -163,6 +163,8 @@ __global__ void k_spk_flatten(SpkArgs A) {
   if ((int)threadIdx.x == __ffs(same) - 1 && __ldcg(A.size + r) < p.it->min_area) atomicAdd(A.size + r, __popc(same));
 }
 
+#define PS_SPK_WARP_KEYS 2048  // a component of more keys is a whole CTA's work
+
 // The small components' cost keys, each component's in one run of A.hi: first a run per root, then the keys.
 __global__ void k_spk_runs(SpkArgs A) {
   Px p;
@@ -183,17 +185,32 @@ __global__ void k_spk_runs(SpkArgs A) {
   base = __shfl_sync(0xffffffffu, base, 31);
   if (n > 0) A.lo[p.g] = base + (unsigned)(sum - n);
 }
+template <bool BIG>
 __global__ void k_spk_keys(SpkArgs A) {
   Px p;
-  if (!spk_px(A, p)) return;
-  const int r = A.parent[p.g];
-  if (r < 0) return;
-  const int n = A.size[r];
-  if (n > 1 && n < p.it->min_area) A.hi[A.lo[r] + atomicAdd(A.cnt + r, 1u)] = fkey(A.cost[p.g]);
+  const bool in = spk_px(A, p);
+  const int r = in ? A.parent[p.g] : -1;
+  const int n = r >= 0 ? A.size[r] : 0;
+  const bool put = n > 1 && n < p.it->min_area;
+  // one addition per key on the component's cursor, per warp on a large component's (its keys would queue up on it)
+  const bool big = BIG && put && n > PS_SPK_WARP_KEYS;
+  const unsigned act = BIG ? __ballot_sync(0xffffffffu, big) : 0u;
+  if (!put) return;
+  unsigned at;
+  if (big) {
+    const unsigned same = __match_any_sync(act, r);
+    const int lead = __ffs(same) - 1;
+    at = 0u;
+    if ((int)threadIdx.x == lead) at = atomicAdd(A.cnt + r, (unsigned)__popc(same));
+    at = __shfl_sync(same, at, lead) + __popc(same & ((1u << threadIdx.x) - 1u));
+  } else {
+    at = atomicAdd(A.cnt + r, 1u);
+  }
+  A.hi[A.lo[r] + at] = fkey(A.cost[p.g]);
 }
 
-// The lower median key (the (size/2)-th smallest) of every small component, into A.cnt of its root: the warp takes its
-// roots in turn and halves the 2^32 key range 32 times over the component's run.
+// The lower median key (the (size/2)-th smallest) of every small component of up to PS_SPK_WARP_KEYS keys, into A.cnt
+// of its root: the warp takes its roots in turn and halves the 2^32 key range 32 times over the component's run.
 __global__ void k_spk_median(SpkArgs A) {
   Px p;
   const bool in = spk_px(A, p);
@@ -202,7 +219,7 @@ __global__ void k_spk_median(SpkArgs A) {
   unsigned at = 0u;
   if (in && A.parent[p.g] == p.g) {
     n = A.size[p.g];
-    todo = n > 1 && n < p.it->min_area;
+    todo = n > 1 && n < p.it->min_area && n <= PS_SPK_WARP_KEYS;
     if (todo) at = A.lo[p.g];
     else if (n == 1) A.cnt[p.g] = fkey(A.cost[p.g]);
   }
@@ -222,6 +239,48 @@ __global__ void k_spk_median(SpkArgs A) {
       else lo = mid + 1u;
     }
     if ((int)threadIdx.x == src) A.cnt[p.g] = lo;
+  }
+}
+
+// The same for the components of more keys, each by a whole CTA: one warp's loads would wait for each other (the whole
+// removal, ms, by one warp and one addition per key on the cursor, then so: one component of 1920 × 1080 95.7 -> 8.0,
+// components of 256 × 256 pixels 4.05 -> 1.08, 3 views of one 640 × 480 component each 14.4 -> 1.4).
+__global__ void __launch_bounds__(256) k_spk_median_big(SpkArgs A) {
+  __shared__ int roots[256];
+  __shared__ int nroots;
+  __shared__ int part[8];
+  const int tid = threadIdx.y * 32 + threadIdx.x;
+  Px p;
+  bool big = false;
+  if (spk_px(A, p) && A.parent[p.g] == p.g) {
+    const int n = A.size[p.g];
+    big = n > PS_SPK_WARP_KEYS && n < p.it->min_area;
+  }
+  if (!__syncthreads_or(big)) return;
+  if (tid == 0) nroots = 0;
+  __syncthreads();
+  if (big) roots[atomicAdd(&nroots, 1)] = p.g;
+  __syncthreads();
+  for (int i = 0; i < nroots; ++i) {  // in any order: each writes its own root's word
+    const int len = A.size[roots[i]];
+    const unsigned* run = A.hi + A.lo[roots[i]];
+    unsigned lo = 0u, hi = 0xFFFFFFFFu;
+    for (int it = 0; it < 32; ++it) {
+      const unsigned mid = lo + (hi - lo) / 2u;
+      int c = 0;
+#pragma unroll 8
+      for (int k = tid; k < len; k += 256) c += run[k] <= mid;
+      c = __reduce_add_sync(0xffffffffu, c);
+      if (threadIdx.x == 0) part[threadIdx.y] = c;
+      __syncthreads();
+      int sum = 0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum += part[k];
+      __syncthreads();  // before the next halving writes part
+      if (sum >= len / 2 + 1) hi = mid;
+      else lo = mid + 1u;
+    }
+    if (tid == 0) A.cnt[roots[i]] = lo;
   }
 }
 
@@ -260,10 +319,16 @@ cudaError_t launch_speckles(const SpkArgs& A, int ntiles, cudaStream_t st, int* 
   k_spk_border<<<ntiles, b, 0, st>>>(A);
   k_spk_flatten<<<ntiles, b, 0, st>>>(A);
   k_spk_runs<<<ntiles, b, 0, st>>>(A);
-  k_spk_keys<<<ntiles, b, 0, st>>>(A);
+  // Components of more than PS_SPK_WARP_KEYS keys are small only under a limit above that, which the default limit (2e-4
+  // of the view) is from 10 Mpixel on.
+  bool big = false;
+  for (int i = 0; i < A.nitems; ++i) big = big || A.items[i].min_area > PS_SPK_WARP_KEYS + 1;
+  if (big) k_spk_keys<true><<<ntiles, b, 0, st>>>(A);
+  else k_spk_keys<false><<<ntiles, b, 0, st>>>(A);
   k_spk_median<<<ntiles, b, 0, st>>>(A);
+  if (big) k_spk_median_big<<<ntiles, b, 0, st>>>(A);
   k_spk_erase<<<ntiles, b, 0, st>>>(A);
-  *launches += 7;
+  *launches += big ? 8 : 7;
   return cudaGetLastError();
 }
 

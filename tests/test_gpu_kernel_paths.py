@@ -92,6 +92,44 @@ def test_speckles_at_tile_edges(w, h, frac):
     assert removed == n
 
 
+@pytest.mark.parametrize("w,sizes", [(64, [2047, 2048, 2049, 2050]), (64, [2049, 300, 5001]), (257, [40000, 2049, 70000])])
+def test_speckles_of_large_components(w, sizes):
+    """Components on both sides of what one warp takes, in row-major runs of pixels.  Of each, the keys up to the limit are
+    just not enough, or just enough, to hold the lower median: an error of one key in either direction shows."""
+    total = sum(sizes)
+    h = -(-total // w)
+    wl = scenes.workload_small(w, h, views=2, window_radius=1, seed=2, sources=1)
+    rng = np.random.default_rng(total)
+    depth, cost = np.zeros(w * h, np.float32), np.full(w * h, 2.0, np.float32)
+    expect, o = np.zeros(w * h, bool), 0
+    for i, n in enumerate(sizes):
+        depth[o:o + n] = (30.0, 40.0)[i % 2]
+        low = n // 2 + i % 2
+        cost[o:o + n] = rng.permutation(np.r_[rng.choice([0.125, 0.5, 1.0], low), rng.choice([1.125, 1.5], n - low)])
+        expect[o:o + n] = i % 2 == 0
+        o += n
+    states = []
+    for k in range(2):
+        st = ViewState.new(w, h)
+        st.depth[...], st.cost[...], st.normal[..., 2] = depth.reshape(h, w), cost.reshape(h, w), -1.0
+        states.append(st)
+    post = fusion.default_post()
+    post.speckle_min_area_frac, post.speckle_keep_cost = 1.5, 1.0
+    be = PatchMatchBackend(0)
+    with be.begin(wl.input) as s:
+        s.upload(0, wl.views, states)
+        s.median_filter(wl.input, 0, wl.views, states)  # its input stays in the readout planes
+        removed = s.postprocess_resident(0, wl.views, post)
+        after = s.readout_download(0, wl.views)
+    be.close()
+    d, nn = states[0].depth.copy(), states[0].normal.copy()
+    assert oracle.remove_speckles(d, nn, states[0].cost, post) * 2 == removed == 2 * expect.sum()
+    np.testing.assert_array_equal((d == 0).ravel()[:total], expect[:total])
+    for a in after:
+        np.testing.assert_array_equal(a.depth, d)
+        np.testing.assert_array_equal(a.normal, nn)
+
+
 @pytest.mark.parametrize("repeat,max_batch", [([0, 0], 64), ([1, 0, 1, 1, 2, 0], 64), ([0, 1, 0, 2, 2], 2)])
 def test_speckles_of_views_named_more_than_once(repeat, max_batch):
     """Within one launch and across launches: each view is cleaned once, and its erased pixels count once."""
