@@ -61,6 +61,19 @@ def test_weight_gradient_tiles_match_fp64(shape):
     assert (np.abs(dw - ref) <= b * h * w * 2.0 ** -23 * mag + 1e-30).all()
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1, 8, 8), (2, 8, 16, 32, 64), (1, 9, 17, 40, 24), (3, 25, 33, 96, 48),
+                                   (1, 70, 130, 56, 128), (5, 3, 40, 224, 16), (2, 64, 129, 32, 16)])
+def test_weight_gradient_counts_every_pixel_once(shape):
+    """Inputs and gradients in {-1, 0, 1}: every product and partial sum is a whole number below 2^24, exact in binary32
+    in any order, so a pixel left out or taken twice anywhere shows, whatever the number of pixels."""
+    b, h, w, ci, co = shape
+    rng = np.random.default_rng(70 + sum(shape))
+    x, dy = (rng.integers(-1, 2, (b, h, w, c)).astype(np.float32) for c in (ci, co))
+    _, _, dw = proposal.conv_check(O.bf16_bits(x), np.zeros((co, 9, ci), np.float32), O.bf16_bits(dy))
+    _, ref, _ = O.conv_grads(x, np.zeros((co, 9, ci)), dy)
+    np.testing.assert_array_equal(dw, ref)
+
+
 def _labels(rng, b, h, w, dr=(25.0, 60.0)):
     lab = np.zeros((b, h, w, 6), np.float32)
     lab[..., 0] = rng.uniform(0, 1, (b, h, w))
@@ -120,7 +133,8 @@ def test_network_gradients_match_fp64_oracle():
 
 @pytest.mark.parametrize("wr,size,tuning", [(3, (64, 48), 0), (6, (80, 64), 0), (6, (80, 64), 6), (3, (64, 48), 2)])
 def test_sweep_bitwise_vs_oracle(wr, size, tuning):
-    """Software bilinear (tuning 0) and texture-gather sampling (tuning with PS_TUNE_TEX_GATHER) give the same bits."""
+    """The sweep kernel of the windows 13x13 and the one for any other window (radius 3), under the default tuning word and
+    under two words that select the same gathers."""
     wl = scenes.workload_small(size[0], size[1], views=3, window_radius=wr, seed=11)
     be = PatchMatchBackend(0, math="parity", tuning=tuning)
     w, h = size
