@@ -1,6 +1,6 @@
 """Device paths at the sizes where they can go wrong, against the CPU oracle bit for bit: windows without a kernel of their
-own, the costs a run keeps (more sources than it keeps, planes without depth), the speckle tiles' edges, the median's,
-downloads beside running work."""
+own, the longest image sides, the costs a run keeps (more sources than it keeps, planes without depth), the speckle
+tiles' edges and large components, the median's edges, downloads beside running work."""
 import numpy as np
 import pytest
 
@@ -37,6 +37,28 @@ def test_uncompiled_windows_default_tuning(wr, ws):
     be.close()
     for a, b in zip(gpu, cpu):
         _same(a, b, f"window {wr},{ws}")
+
+
+@pytest.mark.parametrize("w,h,f32", [(32768, 12, False), (11, 32768, True), (16385, 9, True)])
+def test_largest_image_sides(w, h, f32):
+    """The longest sides a session takes: a gather's integer coordinate selects the same footprint at texel 32767 as at 0,
+    also where the footprint leaves the image at either end."""
+    k, step = (28000.0, 28000.0, w / 2.0, h / 2.0), 0.6
+    cams = [scenes.Camera(f"side{i}", k, np.eye(3), np.array([i * step * (w > h), i * step * (h > w), 0.0]), w, h)
+            for i in (-1, 0, 1)]
+    rng = np.random.default_rng(w)
+    img = [rng.random((h, w), np.float32) for _ in cams]
+    inp = scenes.kernel_input(cams, img, [[1, 2], [0, 2], [1]], (25.0, 60.0), window_radius=3, gray8=not f32)
+    p = RunParams(0, False, True, 1, 1)
+    gpu, cpu = [ViewState.new(w, h)], [ViewState.new(w, h)]
+    be = PatchMatchBackend(0)
+    with be.begin(inp) as s:
+        s.run([1], gpu, p)
+        costs = s.evaluate(0, [1], gpu)
+    be.close()
+    oracle.run(inp, [1], cpu, p)
+    _same(gpu[0], cpu[0], f"{w} x {h}")
+    np.testing.assert_array_equal(costs[0], oracle.evaluate(inp, 0, [1], cpu, False)[0])
 
 
 @pytest.mark.parametrize("tuning", [0, 42])
