@@ -314,7 +314,6 @@ const char* site_name(unsigned site) {
   switch (site) {
     case PS_SITE_TILE: return "reference tile";
     case PS_SITE_BOX: return "staged source box";
-    case PS_SITE_PLANE: return "source plane";
     case PS_SITE_STATE: return "state arrays";
     case PS_SITE_SOURCE: return "source view index";
     case PS_SITE_SNAPSHOT: return "depth snapshot";

@@ -47,7 +47,6 @@ enum PsCheckSite {
   PS_SITE_NONE = 0,
   PS_SITE_TILE = 1,      // reference tile in shared memory (window taps, reference statistics)
   PS_SITE_BOX = 2,       // staged source box in shared memory (the footprint bound)
-  PS_SITE_PLANE = 3,     // bordered source plane in global memory (bilinear taps)
   PS_SITE_STATE = 4,     // per-pixel state arrays (plane, cost, best view, prior)
   PS_SITE_SOURCE = 5,    // source view index of a pair
   PS_SITE_SNAPSHOT = 6,  // depth snapshot of a source view (geometric term)

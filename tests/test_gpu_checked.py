@@ -28,8 +28,7 @@ def _same(a, b, what):
         np.testing.assert_array_equal(x.cost, y.cost, err_msg=what)
 
 
-# two lanes per pixel; one lane + texture gather; row pairs + texture gather; staged source boxes + texture gather;
-# row pairs + texture gather in the persistent kernel; staged boxes loaded by TMA + texture gather
+# 0, 6 and 10: the default kernel; 18: staged source boxes; 42: the persistent kernel; 90: staged boxes loaded by TMA
 @pytest.mark.parametrize("tuning", [0, 6, 10, 18, 42, 90])
 def test_checked_kernels_equal_the_oracle(tuning):
     """Random init + photometric iterations, a geometric iteration through a snapshot, then the filter: the checked

@@ -78,9 +78,9 @@ def test_evaluate_photometric_parity(backend):
 
 @pytest.mark.parametrize("wr,ws", [(3, 1), (5, 1), (5, 2), (6, 1), (4, 1)])
 def test_evaluate_and_filter_through_texture_gathers(wr, ws):
-    """A session with texture objects (PS_TUNE_TEX_GATHER) samples the sources of the run-start evaluate, the
-    evaluate call and the filter through texture gathers at the specialised windows (the generic window keeps the
-    plane loads): the same bits as the oracle for photometric and geometric top-K costs and the filter counts."""
+    """The run-start evaluate, the evaluate call and the filter sample the sources through texture gathers, at the windows
+    with kernels of their own and at one without (radius 4): the same bits as the oracle for photometric and geometric
+    top-K costs and the filter counts."""
     from cumulus3d_b200 import _lib
     from cumulus3d_b200.patchstereo import PatchMatchBackend
     wl = scenes.workload_small(96, 64, views=3, window_radius=wr, window_step=ws, seed=70 + wr)
@@ -299,11 +299,12 @@ def test_bit_reproducible(backend):
         _assert_same(x, y, "rerun")
 
 
-# 42: row pairs + gather in the persistent kernel; 88 / 90: staged boxes loaded by TMA (without / with the gather)
+# 1 to 8 and 10: the default kernel under its other words; 16 / 18: staged boxes; 42: the persistent kernel; 88 / 90: staged
+# boxes loaded by TMA
 @pytest.mark.parametrize("tuning", [1, 2, 3, 4, 5, 6, 7, 8, 10, 16, 18, 42, 88, 90])
 def test_half_step_variants_bitwise_equal(tuning):
-    """Every half-step kernel variant (weight cache off, texture gather, one lane per pixel, row-pair f32x2 loops,
-    staged source boxes) gives the oracle's bits."""
+    """Every tuning word that is accepted gives the oracle's bits: the four half-step kernels (default, persistent, staged
+    boxes by cp.async and by TMA) and the words that name one of them a second time."""
     from cumulus3d_b200.patchstereo import PatchMatchBackend
     wl = scenes.workload_small(72, 56, window_radius=6, seed=13)
     p = RunParams(0, False, True, 2, 1)
@@ -320,7 +321,7 @@ def test_half_step_variants_bitwise_equal(tuning):
 @pytest.mark.parametrize("tuning", [8, 10, 16, 18, 42, 88, 90])
 @pytest.mark.parametrize("wr,ws", [(3, 1), (5, 1), (5, 2), (6, 1)])
 def test_row_pair_and_staged_variants_converged(tuning, wr, ws):
-    """The row-pair and staged-box variants on every compiled window, over a photometric run long enough for the
+    """The default, persistent and staged-box kernels on every compiled window, over a photometric run long enough for the
     planes to converge (so that warps' footprints overlap and the staged boxes are used), then a geometric run."""
     from cumulus3d_b200.patchstereo import PatchMatchBackend
     wl = scenes.workload_small(128, 96, views=3, window_radius=wr, window_step=ws, seed=31 + wr)
