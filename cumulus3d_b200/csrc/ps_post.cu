@@ -476,8 +476,12 @@ __device__ void fuse_emit(const FuseArgs& A, const FuseView& cv, int v, int col,
   A.nvis[slot] = (unsigned char)write_vis(A.vis + slot * A.vis_stride, v, hits, nh);
 }
 
-// First pass (fusion.rs:243-333) of view A.v.  A CTA takes a 32 × 32 tile: its pixels with depth that no earlier view used
+// First pass (fusion.rs:243-333) of view A.v.  A CTA takes a 32 × TH tile: its pixels with depth that no earlier view used
 // go into a list first (after the first views they are few and scattered), and one thread evaluates each of the list.
+//
+// The evaluation is a chain of FP64 latencies, so warps per SM count: two CTAs, 128 registers.  (Left to itself the compiler
+// takes 152 and one CTA fits: 24 views of 1920 × 1080 took 21.4 ms so, and 14.0 ms now; a thread per pixel with 128
+// registers and no list 22.3 ms.)
 __device__ void fuse_pixel(const FuseArgs& A, const FuseView& cv, int col, int row) {
   const long long pix = (long long)row * cv.w + col;
   const float4 q = A.plane[cv.off + pix];
@@ -511,14 +515,15 @@ __device__ void fuse_pixel(const FuseArgs& A, const FuseView& cv, int col, int r
   fuse_emit(A, cv, A.v, col, row, P, hits, nh);
 }
 
-__global__ void __launch_bounds__(256) k_fuse(FuseArgs A) {
-  __shared__ unsigned short list[1024];
+template <int TH>
+__global__ void __launch_bounds__(256, 2) k_fuse(FuseArgs A) {
+  __shared__ unsigned short list[32 * TH];
   __shared__ int count;
   const FuseView& cv = A.views[A.v];
-  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, tid = threadIdx.y * 32 + threadIdx.x;
+  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * TH, tid = threadIdx.y * 32 + threadIdx.x;
   if (tid == 0) count = 0;
   __syncthreads();
-  for (int ty = threadIdx.y; ty < 32; ty += 8) {
+  for (int ty = threadIdx.y; ty < TH; ty += 8) {
     const int col = x0 + threadIdx.x, row = y0 + ty;
     bool todo = false;
     if (col < cv.w && row < cv.h) {
@@ -533,6 +538,15 @@ __global__ void __launch_bounds__(256) k_fuse(FuseArgs A) {
   }
   __syncthreads();
   for (int i = tid; i < count; i += 256) fuse_pixel(A, cv, x0 + (list[i] & 31), y0 + (list[i] >> 5));
+}
+
+// Without marks nearly every pixel with depth is evaluated: a thread per pixel, no list (12 views of 960 × 540: 2.9 ms, with
+// the list 3.0 ms).
+__global__ void __launch_bounds__(256, 2) k_fuse_all(FuseArgs A) {
+  const FuseView& cv = A.views[A.v];
+  const int col = blockIdx.x * 32 + threadIdx.x, row = blockIdx.y * 8 + threadIdx.y;
+  if (col >= cv.w || row >= cv.h || !(A.plane[cv.off + (long long)row * cv.w + col].w > 0.0f)) return;
+  fuse_pixel(A, cv, col, row);
 }
 
 // ---- second pass of leftover pixels (fusion.rs:540-627) ------------------------------------------------------
@@ -1071,8 +1085,13 @@ cudaError_t launch_smooth_pass(const SmoothArgs& A, cudaStream_t st) {
 }
 
 cudaError_t launch_fuse(const FuseArgs& A, int w, int h, cudaStream_t st) {
-  const dim3 b(32, 8), g((w + 31) / 32, (h + 31) / 32);
-  k_fuse<<<g, b, 0, st>>>(A);
+  // Tiles of 16 rows pack the marked views' pixels better, tiles of 8 rows leave more CTAs to views of few: 16 from three
+  // waves of two CTAs on 148 SMs on (ms for all views, 8 and 16 rows, marks on: 6 × 161 × 119 0.18 / 0.23, 3 × 640 × 480
+  // 0.155 / 0.166, 12 × 960 × 540 2.19 / 1.76, 6 × 1920 × 1080 2.64 / 2.17).
+  const dim3 b(32, 8), g16((w + 31) / 32, (h + 15) / 16), g8((w + 31) / 32, (h + 7) / 8);
+  if (!A.mark_used) k_fuse_all<<<g8, b, 0, st>>>(A);
+  else if ((long long)g16.x * g16.y >= 3 * 2 * 148) k_fuse<16><<<g16, b, 0, st>>>(A);
+  else k_fuse<8><<<g8, b, 0, st>>>(A);
   return cudaGetLastError();
 }
 

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from cumulus3d_b200 import fusion, scenes
-from cumulus3d_b200.patchstereo import PatchMatchBackend
+from cumulus3d_b200.patchstereo import PatchMatchBackend, ViewState
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -77,6 +77,40 @@ def test_fusion_bitwise_vs_oracle(pipeline):
                         [scenes.unit_plane(kv.levels[0].pixels) for kv in wl.input.views], views[1:], prm)
     assert n2 == len(want2)
     np.testing.assert_array_equal(s.fused_points().keys, want2.keys)
+
+
+@pytest.mark.parametrize("w,h", [(40, 29), (961, 448), (961, 449)])
+@pytest.mark.parametrize("mark", [0, 1])
+def test_fusion_tiles_bitwise_vs_oracle(w, h, mark):
+    """Tiles of 8 rows, and of 16 rows where those make at least 888 (31 x 28 and 31 x 29 for the last two sizes): perturbed
+    true depths, some missing, with and without marks of used pixels."""
+    n = 4
+    cams = scenes.formation(w, h, 2)[:n]
+    img, dep, nrm = scenes.render(cams, 4)
+    src = scenes.nearest_sources(cams, n - 1)
+    inp = scenes.kernel_input(cams, list(img), src, (25.0, 60.0), window_radius=3)
+    rng = np.random.default_rng(w)
+    states = []
+    for v in range(n):
+        st = ViewState.new(w, h)
+        st.depth[...] = np.where(rng.random((h, w)) < 0.1, 0.0, dep[v] * (1 + rng.normal(0, 0.002, (h, w))))
+        st.normal[...], st.cost[...] = nrm[v], rng.uniform(0, 0.5, (h, w))
+        states.append(st)
+    fc = fusion.FusionCams(cams, src)
+    prm = fusion.default_fusion(2)
+    prm.mark_used = mark
+    be = PatchMatchBackend(0)
+    with be.begin(inp) as s:
+        s.upload(0, range(n), states)
+        s.median_filter(inp, 0, range(n), states)  # its input stays in the readout planes
+        count = s.fuse_resident(0, range(n), fc, prm)
+        got = s.fused_points()
+    be.close()
+    want = oracle.fuse(fc, [st.depth for st in states], [st.normal for st in states], [st.cost for st in states],
+                       [scenes.unit_plane(kv.levels[0].pixels) for kv in inp.views], list(range(n)), prm)
+    assert count == len(want) > 0
+    for k in ("keys", "positions", "normals", "colors", "vis_counts"):
+        np.testing.assert_array_equal(getattr(got, k), getattr(want, k), err_msg=k)
 
 
 def test_second_pass_fusion_bitwise_vs_oracle(pipeline):
