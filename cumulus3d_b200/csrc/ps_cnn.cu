@@ -97,7 +97,7 @@ constexpr size_t conv2_smem() {
   return (size_t)2 * (HALO_PX * KCP + 9 * BN * KCP) * sizeof(bf16);
 }
 
-template <int BN>
+template <int BN, bool MASK>
 __global__ void __launch_bounds__(256) k_conv2(ConvArgs a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   bf16* halo = reinterpret_cast<bf16*>(smraw);  // [2][HALO_PX][KCP]
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(256) k_conv2(ConvArgs a) {
         v0 = fmaxf(v0, 0.f);
         v1 = fmaxf(v1, 0.f);
       }
-      if (a.mask) {
+      if (MASK) {
         const __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162*>(a.mask + p * a.cout + co);
         if (!(__low2float(m) > 0.f)) v0 = 0.f;
         if (!(__high2float(m) > 0.f)) v1 = 0.f;
@@ -276,7 +276,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
   return false;
 }
 
-template <int N>
+template <int N, bool MASK>
 __global__ void __launch_bounds__(128, 1) k_conv5(ConvArgs a) {
   using Cfg = Conv5Cfg<N>;
   constexpr int KCH = Cfg::KCH, KG = Cfg::KG, T5_R = Cfg::R;
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(128, 1) k_conv5(ConvArgs a) {
               v[e] = __uint_as_float(v32[j + e]) + (a.bias ? a.bias[c0 + j + e] : 0.f);
               if (a.relu) v[e] = fmaxf(v[e], 0.f);
             }
-            if (a.mask) {
+            if (MASK) {
               const uint4 mq = *reinterpret_cast<const uint4*>(a.mask + p * a.cout + c0 + j);
               const bf16* m = reinterpret_cast<const bf16*>(&mq);
 #pragma unroll
@@ -953,20 +953,22 @@ template <int BN>
 void conv2_launch(const ConvArgs& a, cudaStream_t st) {
   constexpr size_t smem = conv2_smem<BN>();
   // opt-in to more than 48 KB of dynamic shared memory (per device; cheap, so on every launch)
-  ck(cudaFuncSetAttribute(k_conv2<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "conv smem");
+  const auto kern = a.mask ? k_conv2<BN, true> : k_conv2<BN, false>;
+  ck(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "conv smem");
   const long long tiles = (long long)a.B * ((a.H + HT_H - 1) / HT_H) * ((a.W + HT_W - 1) / HT_W);
   dim3 g((unsigned)tiles, (unsigned)((a.cout + BN - 1) / BN));
-  k_conv2<BN><<<g, 256, smem, st>>>(a);
+  kern<<<g, 256, smem, st>>>(a);
 }
 
 template <int N>
 void conv5_launch(const ConvArgs& a, cudaStream_t st) {
   constexpr size_t smem = Conv5Cfg<N>::smem;
   static_assert(smem <= 227 * 1024, "tcgen05 convolution tile exceeds shared memory");
-  ck(cudaFuncSetAttribute(k_conv5<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "conv smem");
+  const auto kern = a.mask ? k_conv5<N, true> : k_conv5<N, false>;
+  ck(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "conv smem");
   constexpr int R = Conv5Cfg<N>::R;
   const long long ctas = (long long)a.B * ((a.H + R - 1) / R) * ((a.W + T5_PX - 1) / T5_PX);
-  k_conv5<N><<<(unsigned)ctas, 128, smem, st>>>(a);
+  kern<<<(unsigned)ctas, 128, smem, st>>>(a);
 }
 
 // 0: tcgen05 for cout in {64, 96, 128} (on B200 the 128 × 32 tile of cout = 32 is faster on mma.sync), 1: mma.sync
