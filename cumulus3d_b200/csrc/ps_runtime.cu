@@ -172,13 +172,19 @@ struct ps_backend {
   cudaMemPool_t pool = nullptr;
   void* pin = nullptr;
   size_t pin_cap = 0;
-  // texture arrays of the previous session, reused by size and format (freeing an array can stall for a long time)
+  // Texture arrays of earlier sessions, reused by size and format.  Making one takes about 0.1 ms, and freeing one can
+  // stall for tens of ms (sessions of two sizes in turn on one backend, begin and end of 6 views of 1920 × 1080: 3.2 ms,
+  // up to 30 ms, when the other size's arrays were freed each time; now 1.2 ms).  The newest session's wait always;
+  // older ones within 1 GiB and a count that keeps the search short.  reclaim() and ps_backend_destroy give them back.
+#define PS_WAITING_ARRAY_BYTES (size_t(1) << 30)
+#define PS_WAITING_ARRAYS 1024
   struct CachedArray {
     cudaArray_t a;
     int w, h;
     bool u8;
+    size_t bytes() const { return (size_t)w * h * (u8 ? 1 : 4); }
   };
-  std::vector<CachedArray> arrays;
+  std::vector<CachedArray> arrays;  // in the order in which their sessions ended
   // host-side failure injection (ps_backend_inject_failure): kind and the successes left before the failure
   uint32_t inject_kind = PS_INJECT_NONE;
   uint32_t inject_after = 0;
@@ -1172,6 +1178,9 @@ int ps_begin(ps_backend* be, const ps_kernel_input* in, ps_session** out) {
       // every u); f32 images are copied from the plane.
       const cudaChannelFormatDesc cdf = cudaCreateChannelDesc<float>();
       const cudaChannelFormatDesc cd8 = cudaCreateChannelDesc<unsigned char>();
+      be->arrays.reserve(be->arrays.size() + (size_t)s->nv * s->nl);  // ps_end appends this session's without allocating
+      s->array_keys.reserve((size_t)s->nv * s->nl);
+      s->arrays.reserve((size_t)s->nv * s->nl);
       for (int v = 0; v < s->nv; ++v)
         for (int l = 0; l < s->nl; ++l) {
           PsLevel& L = lvh[v * s->nl + l];
@@ -1318,9 +1327,18 @@ int ps_end(ps_session* s) {
   for (cudaEvent_t e : s->xfer) cudaEventDestroy(e);
   dfree(s, s->fault);
   for (cudaTextureObject_t t : s->texs) cudaDestroyTextureObject(t);
-  if (s->be) {  // arrays no session reused are freed; this session's arrays wait for the next one
-    for (auto& c : s->be->arrays) cudaFreeArray(c.a);
-    s->be->arrays = s->array_keys;
+  if (s->be) {  // this session's arrays wait for a later one, with earlier sessions' within the bounds
+    auto& wait = s->be->arrays;
+    wait.insert(wait.end(), s->array_keys.begin(), s->array_keys.end());
+    size_t bytes = 0, drop = 0;
+    for (auto& c : wait) bytes += c.bytes();
+    for (; drop + s->array_keys.size() < wait.size() &&
+           (bytes > PS_WAITING_ARRAY_BYTES || wait.size() - drop > PS_WAITING_ARRAYS);
+         ++drop) {
+      bytes -= wait[drop].bytes();
+      cudaFreeArray(wait[drop].a);
+    }
+    wait.erase(wait.begin(), wait.begin() + (long)drop);
   } else {
     for (cudaArray_t a : s->arrays) cudaFreeArray(a);
   }

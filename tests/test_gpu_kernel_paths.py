@@ -1,6 +1,6 @@
 """Device paths at the sizes where they can go wrong, against the CPU oracle bit for bit: windows without a kernel of their
 own, the longest image sides, the costs a run keeps (more sources than it keeps, planes without depth), the speckle
-tiles' edges and large components, the median's edges, downloads beside running work."""
+tiles' edges and large components, the median's edges, downloads beside running work, sessions that reuse texture arrays."""
 import numpy as np
 import pytest
 
@@ -219,4 +219,31 @@ def test_downloads_with_and_without_pending_work(sizes):
                 _same(a, b, "pending, idle")
                 _same(a, c, "pending, filled")
                 assert (a.depth > 0).all()
+    be.close()
+
+
+def test_sessions_of_several_sizes_and_formats_in_turn():
+    """One backend's sessions reuse the texture arrays of earlier ones by size and format: 8-bit and f32 images of one
+    size, another size, and one session with more views than any before."""
+    def workload(w, h, views, f32, seed):
+        wl = scenes.workload_small(w, h, views=views, window_radius=3, seed=seed, positions=2)
+        if f32:
+            wl.input = scenes.kernel_input(wl.cams, [np.asarray(i, np.float32) for i in wl.images],
+                                           [list(v.sources) for v in wl.input.views], (25.0, 60.0), window_radius=3,
+                                           gray8=False)
+        return wl
+    kinds = [workload(64, 40, 3, False, 5), workload(64, 40, 3, True, 6), workload(48, 40, 3, False, 7),
+             workload(64, 40, 5, False, 8)]
+    p = RunParams(0, False, True, 1, 1)
+    want = []
+    for wl in kinds:
+        want.append(_new(wl))
+        oracle.run(wl.input, wl.views, want[-1], p)
+    be = PatchMatchBackend(0)
+    for i in (0, 1, 2, 0, 3, 1, 0, 2, 3, 1):
+        got = _new(kinds[i])
+        with be.begin(kinds[i].input) as s:
+            s.run(kinds[i].views, got, p)
+        for a, b in zip(got, want[i]):
+            _same(a, b, f"session kind {i}")
     be.close()
