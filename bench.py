@@ -229,7 +229,7 @@ def bench_ours(args, rank, world, local):
         if ds:  # the binding resource, from the ncu capture (not measured by this run)
             data_stage = {"resource": "L1 data stage (texture gathers + shared-memory loads)", "busy": ds["busy"],
                           "texture_pipe": ds["texture_pipe_busy"], "lsu_pipe": ds["lsu_pipe_busy"],
-                          "source": "ncu capture of one 6-view launch, profiles/k_half_c2_drone.md"}
+                          "source": "ncu capture of two 6-view launches, profiles/k_half_c2_drone.md"}
     except Exception:
         pass
     res = {

@@ -2,8 +2,8 @@
 
 All variants of the half-step kernel produce the same bits, so the choice only affects speed:
 
-* the default kernel (the words 0, 2, 3, 4, 6, 7, 8 and 10 all select it);
-* staged source boxes (cp.async or TMA tensor loads), a persistent launch per run.
+* the default kernel (the words 0, 2, 3, 4, 6, 7, 8 and 10 all select it, and each is timed by itself);
+* staged source boxes by cp.async (16 and 18) or by TMA tensor loads (90), a persistent launch per run (42).
 
 The tuner times each candidate on a prefix of the caller's own views and returns the fastest tuning word: a
 photometric run of two red-black iterations from random init brings the planes near convergence (the state most

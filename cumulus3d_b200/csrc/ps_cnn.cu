@@ -466,9 +466,12 @@ __global__ void __launch_bounds__(128, 1) k_conv5(ConvArgs a) {
 // and the 9 taps share one copy of X.  The sums stay in FP32 registers over all tiles of the CTA, and are added to dW
 // with one vector reduction per pair at the end.
 //
-// What bounds it is the tensor pipe of mma.sync.  The earlier form (64 × 64 outputs, K chunks of 16 pixels gathered
-// element by element, a division per element) and the one-element kernels around it took a training step of batch 8 at
-// 256 × 256 to 28.5 ms; with this one, masks fused into the convolutions and 16-byte accesses it takes 3.3 ms.
+// What bounds it is latency at two CTAs (18 warps) per SM: the tensor pipe is 32 - 53 % busy while a CTA runs (17 - 43 %
+// of a launch: the last CTAs run alone), and a warp's issues wait for its mma.sync chain (2.7 - 3.4 cycles each) and for
+// the tile's barrier (1.5 - 2.4).  The earlier form (64 × 64 outputs, K chunks of 16 pixels gathered element by element, a
+// division per element) and the one-element kernels around it took a training step of batch 8 at 256 × 256 to 28.5 ms.
+// With this one, masks fused into the convolutions and 16-byte accesses the step's kernels take 2.5 ms; the call, whose
+// host copies and allocations vary from box to box, 3.2 to 6.1 ms.
 struct WgradArgs {
   const bf16* dy;  // [P][cout]
   const bf16* x;   // [B][H][W][cin_stride], or (x2 != null) the half-resolution part of a virtual concatenation

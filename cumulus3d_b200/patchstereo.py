@@ -129,7 +129,8 @@ class DepthSnapshot:
 def _out_arrays(sizes, channels: int = 1, dtype=np.float32, block_bytes: int = 1 << 24) -> List[np.ndarray]:
     """One uninitialised flat array of w·h·channels values per (w, h), for calls that write all of them.  Fresh memory
     costs a page fault per 4 KB; small views share blocks of up to `block_bytes`, which the allocator backs with large
-    pages (and a kept view keeps at most its block alive)."""
+    pages.  The arrays are views of their block: they do not own their data, and one that is kept keeps its whole block
+    (its state, or up to `block_bytes`) alive; `copy()` gives one that does not."""
     item = np.dtype(dtype).itemsize
     out, i = [], 0
     while i < len(sizes):
