@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(128, 1) k_conv5(ConvArgs a) {
 // with one vector reduction per pair at the end.
 //
 // What bounds it is latency at two CTAs (18 warps) per SM: the tensor pipe is 32 - 53 % busy while a CTA runs (17 - 43 %
-// of a launch: the last CTAs run alone), and a warp's issues wait for its mma.sync chain (2.7 - 3.4 cycles each) and for
+// of a launch: grids of 297 to 308 CTAs leave a few for a second wave), and a warp's issues wait for its mma.sync chain (2.7 - 3.4 cycles each) and for
 // the tile's barrier (1.5 - 2.4).  The earlier form (64 × 64 outputs, K chunks of 16 pixels gathered element by element, a
 // division per element) and the one-element kernels around it took a training step of batch 8 at 256 × 256 to 28.5 ms.
 // With this one, masks fused into the convolutions and 16-byte accesses the step's kernels take 2.5 ms; the call, whose
